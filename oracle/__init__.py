@@ -34,7 +34,7 @@ _D = ctypes.POINTER(ctypes.c_double)
 def build(ref: bool = True) -> None:
     """make the C restatement, and the reference build when its tree exists."""
     subprocess.run(["make", "-s", "-C", HERE, "oracle"], check=True)
-    if ref and os.path.isdir(REF_TREE):
+    if ref and os.path.isfile(os.path.join(REF_TREE, "tasklyapunov.cpp")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={REF_TREE}"], check=True)
 
 
