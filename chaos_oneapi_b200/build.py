@@ -42,6 +42,7 @@ CUDA_UNITS = {
     "order.cu": [],
     "split.cu": [],
     "mlp.cu": [],
+    "mlp_fused.cu": [],
     "trajectory.cu": [],
 }
 CXX_UNITS = ["inputs.cpp"]

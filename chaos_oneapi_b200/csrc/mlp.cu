@@ -26,13 +26,18 @@
 
 #include "../../include/chaos_lyap.h"
 #include "../../include/chaos_lyap_surrogate.h"
+#include "mlp_fused.h"
+#include "umma.cuh"
 
 namespace {
 
 using bf16 = __nv_bfloat16;
-
-constexpr int kFeat = 16;   // input features
-constexpr int kOutPad = 16; // output width padded for the tensor-core tiles
+using namespace chaos::umma;
+using chaos::mlp::kFeat;
+using chaos::mlp::kOutPad;
+using chaos::mlp::silu;
+using chaos::mlp::dsilu;
+using chaos::mlp::FeatureMap;
 
 thread_local std::string g_err;
 int fail(int code, const std::string &m) {
@@ -83,42 +88,6 @@ constexpr int kTcM = 128, kTcN = 128, kTcK = 64;
 constexpr int kTcTileBytes = kTcM * kTcK * 2;                // one operand stage: 16 KB
 constexpr int kTcSmemBytes = 4 * kTcTileBytes + 64;          // A, B x 2 stages + barriers
 constexpr int kTcTmemCols = 128;
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// Shared-memory matrix descriptor of tcgen05.mma: start address, leading
-// byte offset (between core matrices adjacent in K), stride byte offset
-// (between core matrices adjacent in M / N), all in 16-byte units; version
-// 1 (bits 46-47); base offset 0; no swizzle (bits 61-63 = 0).
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo & 0x3FFFFu) >> 4) << 16) |
-         ((uint64_t)((sbo & 0x3FFFFu) >> 4) << 32) | (1ull << 46);
-}
-
-// Instruction descriptor of kind::f16: D in FP32 (bits 4-5 = 1), A and B in
-// BF16 (bits 7-9 = 1, bits 10-12 = 1), both K-major (bits 15, 16 = 0),
-// N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-__device__ __forceinline__ uint32_t umma_instr_desc(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
-         ((uint32_t)(M >> 4) << 24);
-}
-
-// Bounded wait for the phase of `parity` of an mbarrier; false if it gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < (1 << 22); i++) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
 
 // Offset (in elements) of element (r, k) of a rows x 64 stage in the
 // no-swizzle K-major core-matrix layout: core matrix (r / 8, k / 8) at
@@ -242,7 +211,7 @@ __global__ void __launch_bounds__(128) gemm_bf16_tc_kernel(const GemmArgs g) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = umma_instr_desc(kTcM, bn);
+  const uint32_t idesc = instr_desc(kTcM, bn);
 
   bool ok = true;
   const int nkb = (g.K + kTcK - 1) / kTcK;
@@ -260,8 +229,8 @@ __global__ void __launch_bounds__(128) gemm_bf16_tc_kernel(const GemmArgs g) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int slices = (min(kTcK, g.K - k0) + 15) / 16;
       for (int j = 0; j < slices; j++) {
-        const uint64_t ad = umma_smem_desc(smem_u32(as) + j * 256, 128, 1024);
-        const uint64_t bd = umma_smem_desc(smem_u32(bs) + j * 256, 128, 1024);
+        const uint64_t ad = smem_desc(smem_u32(as) + j * 256, 128, 1024);
+        const uint64_t bd = smem_desc(smem_u32(bs) + j * 256, 128, 1024);
         const uint32_t accum = (kb > 0 || j > 0) ? 1u : 0u;
         asm volatile(
             "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -334,26 +303,16 @@ int gemm(GemmArgs g, int nz, cudaStream_t s, int *err) {
 }
 
 // ------------------------------------------------------- elementwise parts
-__device__ __forceinline__ float silu(float z) { return z / (1.f + __expf(-z)); }
-__device__ __forceinline__ float dsilu(float z) {
-  const float sg = 1.f / (1.f + __expf(-z));
-  return sg * (1.f + z * (1.f - sg));
-}
-
-// 16 Fourier features of the normalised point (shared by all networks):
-// sin and cos of 2 pi (w_f . (u, v)) for 8 frequency vectors w_f.
-struct Freqs {
-  float w[8][2];
-};
-__global__ void features_kernel(const double *xy, int64_t N, double u0, double us, double v0,
-                                double vs, Freqs fr, bf16 *X) {
+// 16 Fourier features of the normalised point (shared by all networks).
+__global__ void features_kernel(const double *xy, int64_t N, FeatureMap fm, bf16 *X) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const float u = (float)((xy[2 * i] - u0) * us), v = (float)((xy[2 * i + 1] - v0) * vs);
+  float u, v;
+  chaos::mlp::normalised(fm, xy, i, u, v);
 #pragma unroll
   for (int f = 0; f < 8; f++) {
     float sn, cs;
-    sincospif(2.f * (fr.w[f][0] * u + fr.w[f][1] * v), &sn, &cs);
+    chaos::mlp::feature_pair(fm, u, v, f, sn, cs);
     X[i * kFeat + 2 * f] = __float2bfloat16(sn);
     X[i * kFeat + 2 * f + 1] = __float2bfloat16(cs);
   }
@@ -422,13 +381,10 @@ __global__ void adam_kernel(float *p, const float *gr, float *m, float *v, bf16 
                             float lr, float b1, float b2, float eps, float c1, float c2) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float g = gr[i];
-  const float mi = b1 * m[i] + (1.f - b1) * g;
-  const float vi = b2 * v[i] + (1.f - b2) * g * g;
+  float mi = m[i], vi = v[i];
+  p[i] = chaos::mlp::adam_update(p[i], gr[i], mi, vi, lr, b1, b2, eps, c1, c2);
   m[i] = mi;
   v[i] = vi;
-  const float upd = lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  p[i] -= upd;
   pb[i] = __float2bfloat16(p[i]);
 }
 
@@ -444,20 +400,24 @@ __global__ void gather_batch_kernel(const int *idx, int64_t B, const double *xy,
   for (int c = 0; c < outs; c++) Tb[r * outs + c] = (float)T[j * outs + c];
 }
 
-__global__ void to_bf16_kernel(const float *p, bf16 *pb, int64_t n) {
+// BF16 copy of n parameters, np per network, in the kernels' order.
+__global__ void to_bf16_kernel(const float *p, bf16 *pb, int64_t n, int64_t np,
+                               chaos::mlp::BfOrder order) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) pb[i] = __float2bfloat16(p[i]);
+  if (i < n) pb[i / np * np + order.at(i % np)] = __float2bfloat16(p[i]);
 }
 
-// Ensemble mean and standard deviation (de-standardised) of the outputs.
-__global__ void ensemble_kernel(const float *Y, int E, int64_t rows, int outs, const float *tmean,
+// Ensemble mean and standard deviation (de-standardised) of the outputs; a
+// row of Y is `ys` floats.
+__global__ void ensemble_kernel(const float *Y, int ys, int E, int64_t rows, int outs,
+                                const float *tmean,
                                 const float *tstd, float *mean, float *std) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rows) return;
   for (int c = 0; c < outs; c++) {
     float s = 0.f, s2 = 0.f;
     for (int z = 0; z < E; z++) {
-      const float y = Y[(z * rows + r) * kOutPad + c] * tstd[c] + tmean[c];
+      const float y = Y[(z * rows + r) * ys + c] * tstd[c] + tmean[c];
       s += y;
       s2 += y * y;
     }
@@ -483,7 +443,7 @@ struct chaos_mlp {
   float tmean[kOutPad], tstd[kOutPad];
   float *d_tmean = nullptr, *d_tstd = nullptr, *d_tinv = nullptr;
   double u0 = 0, us = 1, v0 = 0, vs = 1;
-  Freqs freqs;    // feature frequencies (cycles over the unit box)
+  chaos::mlp::Freqs freqs;  // feature frequencies (cycles over the unit box)
   int64_t t = 0;  // Adam step
   // workspace for `cap` rows
   int64_t cap = 0;
@@ -494,6 +454,32 @@ struct chaos_mlp {
   int *idx = nullptr;      // minibatch row indices of kTrainChunk steps
   int64_t idx_cap = 0;
   int *d_err = nullptr;  // set by a GEMM whose wait on the tensor core gave up
+  // fused kernels (W = 64, 128): minibatch tiles, outputs of a prediction chunk
+  chaos::mlp::TrainBuffers fb = {};
+  int64_t fb_tiles = 0;
+  float *Yp = nullptr;
+  int64_t yp_cap = 0;
+
+  bool fused() const { return chaos::mlp::fused_width(W); }
+  FeatureMap features() const { return FeatureMap{u0, us, v0, vs, freqs}; }
+  chaos::mlp::BfOrder order() const {
+    chaos::mlp::BfOrder o{};
+    o.W = W;
+    const int64_t w = W, size[4] = {kFeat * w, w * w, w * w, w * kOutPad};
+    for (int l = 0; l < 4; l++) {
+      o.off_w[l] = off_w[l];
+      o.size_w[l] = size[l];
+      o.cols[l] = l < 3 ? W : kOutPad;
+    }
+    return o;
+  }
+  chaos::mlp::Params params() const {
+    chaos::mlp::Params q{};
+    q.E = E, q.W = W, q.outs = outs, q.np = np;
+    for (int l = 0; l < 4; l++) q.off_w[l] = off_w[l], q.off_b[l] = off_b[l];
+    q.p = p, q.pb = pb, q.g = g, q.m = m, q.v = v, q.err = d_err;
+    return q;
+  }
 };
 
 namespace {
@@ -534,6 +520,54 @@ int ensure_ws(chaos_mlp *h, int64_t rows) {
     return fail(CHAOS_LYAP_ENOMEM, std::string("surrogate workspace: ") + cudaGetErrorString(e));
   }
   h->cap = rows;
+  return 0;
+}
+
+void free_fused(chaos_mlp *h) {
+  cudaFree(h->fb.X);
+  cudaFree(h->fb.dY);
+  for (int l = 0; l < 3; l++) {
+    cudaFree(h->fb.A[l]);
+    cudaFree(h->fb.dZ[l]);
+  }
+  h->fb = chaos::mlp::TrainBuffers{};
+  h->fb_tiles = 0;
+}
+
+// Minibatch tiles of the fused training kernels for `rows` rows.
+int ensure_fused(chaos_mlp *h, int64_t rows) {
+  const int64_t tiles = chaos::mlp::train_tiles(rows);
+  if (tiles <= h->fb_tiles) return 0;
+  free_fused(h);
+  cudaError_t e = cudaSuccess;
+  auto al = [&](bf16 **p, int64_t n) {
+    if (e == cudaSuccess) e = cudaMalloc((void **)p, sizeof(bf16) * n * tiles * 128);
+  };
+  al(&h->fb.X, kFeat);
+  al(&h->fb.dY, (int64_t)h->E * kOutPad);
+  for (int l = 0; l < 3; l++) {
+    al(&h->fb.A[l], (int64_t)h->E * h->W);
+    al(&h->fb.dZ[l], (int64_t)h->E * h->W);
+  }
+  if (e != cudaSuccess) {
+    free_fused(h);
+    return fail(CHAOS_LYAP_ENOMEM, std::string("surrogate workspace: ") + cudaGetErrorString(e));
+  }
+  h->fb_tiles = tiles;
+  return 0;
+}
+
+// Outputs of `rows` rows of every network.
+int ensure_outputs(chaos_mlp *h, int64_t rows) {
+  if (rows <= h->yp_cap) return 0;
+  cudaFree(h->Yp);
+  h->Yp = nullptr;
+  h->yp_cap = 0;
+  const int64_t ys = (h->outs + 3) / 4 * 4;
+  cudaError_t e = cudaMalloc((void **)&h->Yp, sizeof(float) * h->E * rows * ys);
+  if (e != cudaSuccess)
+    return fail(CHAOS_LYAP_ENOMEM, std::string("surrogate workspace: ") + cudaGetErrorString(e));
+  h->yp_cap = rows;
   return 0;
 }
 
@@ -592,8 +626,7 @@ int backward(chaos_mlp *h, int64_t rows, cudaStream_t s) {
 
 // One forward / backward on `rows` points starting at xy / T (device).
 int grad_step(chaos_mlp *h, const double *xy, const float *T, int64_t rows, cudaStream_t s) {
-  features_kernel<<<blocks(rows, 256), 256, 0, s>>>(xy, rows, h->u0, h->us, h->v0, h->vs, h->freqs,
-                                                    h->X);
+  features_kernel<<<blocks(rows, 256), 256, 0, s>>>(xy, rows, h->features(), h->X);
   int rc = forward(h, rows, s);
   if (rc) return rc;
   cudaMemsetAsync(h->loss, 0, sizeof(float) * h->E, s);
@@ -708,7 +741,7 @@ int chaos_mlp_create(int ensemble, int width, int outputs, uint64_t seed, int de
   cudaMemset(h->m, 0, sizeof(float) * n);
   cudaMemset(h->v, 0, sizeof(float) * n);
   cudaMemset(h->d_err, 0, sizeof(int));
-  to_bf16_kernel<<<blocks(n, 256), 256>>>(h->p, h->pb, n);
+  to_bf16_kernel<<<blocks(n, 256), 256>>>(h->p, h->pb, n, h->np, h->order());
   for (int c = 0; c < kOutPad; c++) h->tmean[c] = 0.f, h->tstd[c] = 1.f;
   float tb[3 * kOutPad];
   for (int c = 0; c < kOutPad; c++) tb[c] = 0.f, tb[kOutPad + c] = 1.f, tb[2 * kOutPad + c] = 1.f;
@@ -726,6 +759,8 @@ int chaos_mlp_destroy(chaos_mlp *h) {
   DevGuard g(h->device);
   cudaDeviceSynchronize();
   free_ws(h);
+  free_fused(h);
+  cudaFree(h->Yp);
   cudaFree(h->idx);
   cudaFree(h->p);
   cudaFree(h->g);
@@ -800,7 +835,7 @@ int chaos_mlp_set_params(chaos_mlp *h, const float *host) {
   const int64_t n = h->np * h->E;
   cudaError_t e = cudaMemcpy(h->p, host, sizeof(float) * n, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(e, "set_params");
-  to_bf16_kernel<<<blocks(n, 256), 256>>>(h->p, h->pb, n);
+  to_bf16_kernel<<<blocks(n, 256), 256>>>(h->p, h->pb, n, h->np, h->order());
   e = cudaDeviceSynchronize();
   return e == cudaSuccess ? CHAOS_LYAP_OK : cuda_fail(e, "set_params");
 }
@@ -812,13 +847,20 @@ int chaos_mlp_gradient(chaos_mlp *h, const double *xy, const double *T, int64_t 
                        float *grads_out, float *loss_out) {
   if (!h || !xy || !T || rows <= 0) return fail(CHAOS_LYAP_EINVAL, "bad arguments");
   DevGuard g(h->device);
-  int rc = ensure_ws(h, rows);
-  if (rc) return rc;
-  std::vector<double> td(rows * h->outs);
-  cudaMemcpy(td.data(), T, sizeof(double) * td.size(), cudaMemcpyDeviceToHost);
-  std::vector<float> tf(td.begin(), td.end());
-  cudaMemcpy(h->Tb, tf.data(), sizeof(float) * tf.size(), cudaMemcpyHostToDevice);
-  rc = grad_step(h, xy, h->Tb, rows, 0);
+  int rc = 0;
+  if (h->fused()) {
+    if ((rc = ensure_fused(h, rows))) return rc;
+    cudaMemsetAsync(h->loss, 0, sizeof(float) * h->E, 0);
+    rc = chaos::mlp::fused_gradient(h->params(), h->features(), xy, T, nullptr, rows, h->d_tmean,
+                                    h->d_tinv, h->fb, nullptr, h->loss, 0);
+  } else {
+    if ((rc = ensure_ws(h, rows))) return rc;
+    std::vector<double> td(rows * h->outs);
+    cudaMemcpy(td.data(), T, sizeof(double) * td.size(), cudaMemcpyDeviceToHost);
+    std::vector<float> tf(td.begin(), td.end());
+    cudaMemcpy(h->Tb, tf.data(), sizeof(float) * tf.size(), cudaMemcpyHostToDevice);
+    rc = grad_step(h, xy, h->Tb, rows, 0);
+  }
   if (rc) return cuda_fail((cudaError_t)rc, "gradient");
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return cuda_fail(e, "gradient");
@@ -841,15 +883,16 @@ int chaos_mlp_train(chaos_mlp *h, const double *xy, const double *T, int64_t N, 
   DevGuard g(h->device);
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t B = std::min<int64_t>(batch, N);
-  int rc = ensure_ws(h, B);
+  const bool fused = h->fused();
+  int rc = fused ? ensure_fused(h, B) : ensure_ws(h, B);
   if (rc) return rc;
   // The minibatches are drawn on the host (a seeded Fisher-Yates shuffle per
-  // epoch), kTrainChunk steps of row indices at a time, and gathered on the
-  // device from the training set where it lies: a step is three kernels
-  // and a copy of nothing, and the host never waits for the GPU until the
-  // end (each index chunk is copied on the stream, after the steps that read
-  // the previous one).
-  constexpr int kTrainChunk = 256;
+  // epoch), a chunk of steps' row indices at a time, and gathered on the
+  // device from the training set where it lies; the host never waits for the
+  // GPU until the end (each index chunk is copied on the stream, after the
+  // steps that read the previous one).  A chunk is at most 64 KB of indices
+  // (and 256 steps): the next one is drawn while the GPU runs this one.
+  const int kTrainChunk = (int)std::max<int64_t>(1, std::min<int64_t>(256, 16384 / B));
   if (h->idx_cap < kTrainChunk * B) {
     cudaFree(h->idx);
     h->idx = nullptr;
@@ -885,14 +928,24 @@ int chaos_mlp_train(chaos_mlp *h, const double *xy, const double *T, int64_t N, 
                                     cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_fail(e, "batch indices");
     for (int k = 0; k < cs; k++) {
-      gather_batch_kernel<<<blocks(B, 256), 256, 0, s>>>(h->idx + (int64_t)k * B, B, xy, T, h->outs,
-                                                         h->xyb, h->Tb);
-      rc = grad_step(h, h->xyb, h->Tb, B, s);
-      if (rc) return cuda_fail((cudaError_t)rc, "train step");
       h->t++;
       const float b1 = 0.9f, b2 = 0.999f;
       const float c1 = 1.f / (1.f - std::pow(b1, (float)h->t));
       const float c2 = 1.f / (1.f - std::pow(b2, (float)h->t));
+      if (fused) {  // two kernels: forward and backward, weight gradients with Adam
+        const bool last = it0 + k == steps - 1;  // the step whose losses are returned
+        if (last) cudaMemsetAsync(h->loss, 0, sizeof(float) * h->E, s);
+        const chaos::mlp::AdamStep adam{lr, b1, b2, 1e-8f, c1, c2};
+        rc = chaos::mlp::fused_gradient(h->params(), h->features(), xy, T,
+                                        h->idx + (int64_t)k * B, B, h->d_tmean, h->d_tinv, h->fb,
+                                        &adam, last ? h->loss : nullptr, s);
+        if (rc) return cuda_fail((cudaError_t)rc, "train step");
+        continue;
+      }
+      gather_batch_kernel<<<blocks(B, 256), 256, 0, s>>>(h->idx + (int64_t)k * B, B, xy, T, h->outs,
+                                                         h->xyb, h->Tb);
+      rc = grad_step(h, h->xyb, h->Tb, B, s);
+      if (rc) return cuda_fail((cudaError_t)rc, "train step");
       adam_kernel<<<blocks(n, 256), 256, 0, s>>>(h->p, h->g, h->m, h->v, h->pb, n, lr, b1, b2,
                                                  1e-8f, c1, c2);
     }
@@ -912,19 +965,27 @@ int chaos_mlp_predict(chaos_mlp *h, const double *xy, int64_t N, float *mean, fl
   if (!h || !xy || N < 0) return fail(CHAOS_LYAP_EINVAL, "bad arguments");
   DevGuard g(h->device);
   cudaStream_t s = (cudaStream_t)stream;
-  const int64_t chunk = std::min<int64_t>(N, 1 << 16);
-  int rc = ensure_ws(h, std::max<int64_t>(chunk, 1));
+  const bool fused = h->fused();
+  const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(N, fused ? 1 << 18 : 1 << 16));
+  int rc = fused ? ensure_outputs(h, chunk) : ensure_ws(h, chunk);
   if (rc) return rc;
   for (int64_t o = 0; o < N; o += chunk) {
     const int64_t rows = std::min(chunk, N - o);
-    features_kernel<<<blocks(rows, 256), 256, 0, s>>>(xy + 2 * o, rows, h->u0, h->us, h->v0,
-                                                      h->vs, h->freqs, h->X);
-    rc = forward(h, rows, s);
-    if (rc) return cuda_fail((cudaError_t)rc, "predict");
-    output_kernel<<<dim3(blocks(rows, 128), 1, h->E), 128, 0, s>>>(
-        h->Y, h->p + h->off_b[3], h->np, rows, h->outs, nullptr, nullptr, nullptr, nullptr, nullptr);
+    const float *Y = fused ? h->Yp : h->Y;
+    const int ys = fused ? (h->outs + 3) / 4 * 4 : kOutPad;
+    if (fused) {
+      rc = chaos::mlp::fused_predict(h->params(), h->features(), xy + 2 * o, rows, h->Yp, s);
+      if (rc) return cuda_fail((cudaError_t)rc, "predict");
+    } else {
+      features_kernel<<<blocks(rows, 256), 256, 0, s>>>(xy + 2 * o, rows, h->features(), h->X);
+      rc = forward(h, rows, s);
+      if (rc) return cuda_fail((cudaError_t)rc, "predict");
+      output_kernel<<<dim3(blocks(rows, 128), 1, h->E), 128, 0, s>>>(
+          h->Y, h->p + h->off_b[3], h->np, rows, h->outs, nullptr, nullptr, nullptr, nullptr,
+          nullptr);
+    }
     ensemble_kernel<<<blocks(rows, 128), 128, 0, s>>>(
-        h->Y, h->E, rows, h->outs, h->d_tmean, h->d_tstd, mean ? mean + o * h->outs : nullptr,
+        Y, ys, h->E, rows, h->outs, h->d_tmean, h->d_tstd, mean ? mean + o * h->outs : nullptr,
         stdev ? stdev + o * h->outs : nullptr);
   }
   cudaError_t e = cudaStreamSynchronize(s);
