@@ -26,6 +26,21 @@ __device__ __forceinline__ int64_t next_point(const AdaptiveArgs &a) {
   return (int64_t)((q * (unsigned long long)a.queue_stride) % (unsigned long long)a.P);
 }
 
+// RESUME: the next point that has an averaging phase left (points that ended in
+// their transient are in the order too).
+template <bool RESUME> __device__ __forceinline__ int64_t next_open_point(const AdaptiveArgs &a) {
+  int64_t pt = next_point(a);
+  if (RESUME)
+    while (pt < a.P && a.resume.steps[pt] < 0) pt = next_point(a);
+  return pt;
+}
+template <bool RESUME, class M, int K, class R, int INTEG>
+__device__ __forceinline__ void lane_begin(Lane<M, K, R, INTEG> &L, const AdaptiveArgs &a,
+                                           int64_t pt) {
+  if constexpr (RESUME) lane_resume(L, a, pt);
+  else lane_start(L, a, pt);
+}
+
 // Each lane owns one point at a time and runs it as a state machine (one
 // step attempt per loop iteration), so a lane never waits for another lane's
 // phase or renormalisation interval to end: when its point is done it takes
@@ -35,70 +50,113 @@ __device__ __forceinline__ int64_t next_point(const AdaptiveArgs &a) {
 // MINB: resident 128-thread blocks per SM the kernel is compiled for (a
 // register cap: 4 -> 128 registers, 5 -> 96 with a few spills); the
 // autotuner picks the variant.
-template <class M, int K, class R, int INTEG, int MINB>
+// RESUME: the averaging phases of points whose transients have run.
+template <class M, int K, class R, int INTEG, int MINB, bool RESUME = false>
 __global__ void __launch_bounds__(128, MINB) sweep_kernel(const AdaptiveArgs a) {
   const Ctl &c = a.ctl;
   Lane<M, K, R, INTEG> L;
-  int64_t pt = a.queue ? next_point(a) : (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int64_t pt = a.queue ? next_open_point<RESUME>(a) : (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool active = pt < a.P;
-  if (active) lane_start(L, a, pt);
+  if (active) lane_begin<RESUME>(L, a, pt);
   while (__any_sync(0xffffffffu, active)) {
     if (active && lane_step(L, a, c) == kFinished) {
-      pt = a.queue ? next_point(a) : a.P;
+      pt = a.queue ? next_open_point<RESUME>(a) : a.P;
       active = pt < a.P;
-      if (active) lane_start(L, a, pt);
+      if (active) lane_begin<RESUME>(L, a, pt);
     }
     const bool due = active && L.phase != kTransient && L.t_gs >= L.L;
     if (__any_sync(0xffffffffu, due)) {
       if (active && L.phase != kTransient && L.t_gs > 0.f && !lane_gram_schmidt(L, a, c)) {
         lane_finish(L, a, 1);
-        pt = a.queue ? next_point(a) : a.P;
+        pt = a.queue ? next_open_point<RESUME>(a) : a.P;
         active = pt < a.P;
-        if (active) lane_start(L, a, pt);
+        if (active) lane_begin<RESUME>(L, a, pt);
       }
     }
   }
 }
 
+// The transients of all points, one thread each (neighbouring points cost
+// alike), the state alone.
 template <class M, class R, int INTEG>
-int launch_mri(const AdaptiveArgs &a, int block, int persistent_blocks, int variant,
-               cudaStream_t s) {
-  if (a.k != M::N) return kErrUnsupported;
-  auto kern = sweep_kernel<M, M::N, R, INTEG, 1>;
-  if (sizeof(R) == 4) kern = variant == 1 ? sweep_kernel<M, M::N, R, INTEG, 5>
-                                          : sweep_kernel<M, M::N, R, INTEG, 4>;
-  unsigned grid;
-  if (a.queue) {
-    if (persistent_blocks <= 0) {
-      // one full wave: resident blocks per SM x SM count
-      int dev = 0, sms = 0, per_sm = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
-      persistent_blocks = std::max(1, per_sm) * std::max(1, sms);
-    }
-    const int64_t need = (a.P + block - 1) / block;  // never more blocks than points need
-    grid = (unsigned)std::min<int64_t>(persistent_blocks, need);
-  } else {
-    grid = (unsigned)((a.P + block - 1) / block);
+__global__ void __launch_bounds__(128) transient_kernel(const AdaptiveArgs a) {
+  const int64_t pt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pt < a.P) run_transient<M, R, INTEG>(a, a.ctl, pt);
+}
+
+template <class M, class R, int INTEG, bool RESUME> auto sweep_kernel_of(int variant) {
+  if constexpr (sizeof(R) == 4)
+    return variant == 1 ? sweep_kernel<M, M::N, R, INTEG, 5, RESUME>
+                        : sweep_kernel<M, M::N, R, INTEG, 4, RESUME>;
+  else
+    return sweep_kernel<M, M::N, R, INTEG, 1, RESUME>;
+}
+
+// What a launch of one (model, precision, integrator) does.
+struct Launch {
+  enum Kind { kRun, kTransients, kAveraging, kResident } kind;
+  int block, variant;
+  cudaStream_t s;
+  int64_t resident;  // result of kResident: points
+};
+
+// One full wave of blocks: resident blocks per SM x SM count.
+template <class K> int64_t full_wave(K kern, int block) {
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
+  return (int64_t)std::max(1, per_sm) * std::max(1, sms);
+}
+
+template <class M, class R, int INTEG> int launch_mri(const AdaptiveArgs &a, Launch &l) {
+  const auto kern = sweep_kernel_of<M, R, INTEG, false>(l.variant);
+  if (l.kind == Launch::kResident) {
+    l.resident = full_wave(kern, l.block) * l.block;
+    return 0;
   }
+  if (a.k != M::N) return kErrUnsupported;
   AdaptiveArgs ka = a;
   ka.ctl = make_ctl<R>(a);
-  kern<<<grid, block, 0, s>>>(ka);
+  const int64_t need = (a.P + l.block - 1) / l.block;  // never more blocks than points need
+  if (l.kind == Launch::kTransients) {
+    transient_kernel<M, R, INTEG><<<(unsigned)((a.P + 127) / 128), 128, 0, l.s>>>(ka);
+  } else if (l.kind == Launch::kAveraging) {
+    // Few waves: no more blocks than the one-launch form holds (a longest
+    // point's chain of steps, slower the more warps share its scheduler, is
+    // the run); many: every block that fits.
+    const auto resume = sweep_kernel_of<M, R, INTEG, true>(l.variant);
+    const int64_t most = full_wave(resume, l.block), base = full_wave(kern, l.block);
+    const int64_t wave = a.P < 3 * most * l.block ? std::min(most, base) : most;
+    resume<<<(unsigned)std::min(wave, need), l.block, 0, l.s>>>(ka);
+  } else {
+    const int64_t grid = a.queue ? std::min(full_wave(kern, l.block), need) : need;
+    kern<<<(unsigned)grid, l.block, 0, l.s>>>(ka);
+  }
   return (int)cudaGetLastError();
 }
 
-template <class M>
-int launch_m(int integ, int prec, const AdaptiveArgs &a, int block, int pblocks, int variant,
-             cudaStream_t s) {
+template <class M> int launch_m(int integ, int prec, const AdaptiveArgs &a, Launch &l) {
   if (integ == kDverk65) {
-    if (prec == kFP64) return launch_mri<M, double, kDverk65>(a, block, pblocks, variant, s);
-    if (prec == kFP32) return launch_mri<M, float, kDverk65>(a, block, pblocks, variant, s);
+    if (prec == kFP64) return launch_mri<M, double, kDverk65>(a, l);
+    if (prec == kFP32) return launch_mri<M, float, kDverk65>(a, l);
   } else if (integ == kDopri5) {
-    if (prec == kFP64) return launch_mri<M, double, kDopri5>(a, block, pblocks, variant, s);
-    if (prec == kFP32) return launch_mri<M, float, kDopri5>(a, block, pblocks, variant, s);
+    if (prec == kFP64) return launch_mri<M, double, kDopri5>(a, l);
+    if (prec == kFP32) return launch_mri<M, float, kDopri5>(a, l);
   }
   return kErrUnsupported;
+}
+
+int launch_model(int model, int integ, int prec, const AdaptiveArgs &a, Launch &l) {
+  if (l.block <= 0 || l.block > 128 || l.block % 32) l.block = 128;
+  switch (model) {
+    case kShimizu: return launch_m<Shimizu>(integ, prec, a, l);
+    case kLorenz: return launch_m<Lorenz>(integ, prec, a, l);
+    case kRossler: return launch_m<Rossler>(integ, prec, a, l);
+    case kChua: return launch_m<Chua>(integ, prec, a, l);
+    case kHyperRossler: return launch_m<HyperRossler>(integ, prec, a, l);
+    default: return kErrUnsupported;
+  }
 }
 
 // ----------------------------------------------------------- mixed batch
@@ -203,20 +261,31 @@ int launch_batch(int integ, int prec, const BatchArgs &b, int block, cudaStream_
                                   with_ctl(b, prec));
 }
 
-int launch_adaptive(int model, int integ, int prec, const AdaptiveArgs &a, int block,
-                    int persistent_blocks, int variant, cudaStream_t s) {
+int launch_adaptive(int model, int integ, int prec, const AdaptiveArgs &a, int block, int variant,
+                    cudaStream_t s) {
   using namespace adaptive;
   if (a.P <= 0) return 0;
-  if (block <= 0 || block > 128 || block % 32) block = 128;
-  const int pb = persistent_blocks, v = variant;
-  switch (model) {
-    case kShimizu: return launch_m<Shimizu>(integ, prec, a, block, pb, v, s);
-    case kLorenz: return launch_m<Lorenz>(integ, prec, a, block, pb, v, s);
-    case kRossler: return launch_m<Rossler>(integ, prec, a, block, pb, v, s);
-    case kChua: return launch_m<Chua>(integ, prec, a, block, pb, v, s);
-    case kHyperRossler: return launch_m<HyperRossler>(integ, prec, a, block, pb, v, s);
-    default: return kErrUnsupported;
-  }
+  Launch l{Launch::kRun, block, variant, s, 0};
+  return launch_model(model, integ, prec, a, l);
+}
+
+int64_t adaptive_resident(int model, int integ, int prec, int block, int variant) {
+  using namespace adaptive;
+  Launch l{Launch::kResident, block, variant, nullptr, 0};
+  return launch_model(model, integ, prec, AdaptiveArgs{}, l) ? 0 : l.resident;
+}
+
+int launch_adaptive_two_phase(int model, int integ, int prec, const AdaptiveArgs &a, int block,
+                              int variant, void *order_scratch, cudaStream_t s) {
+  using namespace adaptive;
+  if (a.P <= 0) return 0;
+  Launch l{Launch::kTransients, block, variant, s, 0};
+  int rc = launch_model(model, integ, prec, a, l);
+  if (!rc)
+    rc = launch_order_longest_first(a.resume.cost, a.P, const_cast<int32_t *>(a.order),
+                                    order_scratch, s);
+  l.kind = Launch::kAveraging;
+  return rc ? rc : launch_model(model, integ, prec, a, l);
 }
 
 }  // namespace chaos

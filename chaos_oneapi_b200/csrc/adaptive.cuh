@@ -1027,6 +1027,36 @@ CL_HD void lane_start(Lane<M, K, R, INTEG> &L, const AdaptiveArgs &a, int64_t pt
   }
 }
 
+// Starts a point whose transient has run (Resume): what lane_start and the
+// transient's steps would have left in the lane.
+template <class M, int K, class R, int INTEG>
+CL_HD void lane_resume(Lane<M, K, R, INTEG> &L, const AdaptiveArgs &a, int64_t pt) {
+  constexpr int N = M::N;
+  Cold &cs = cold_slot();
+  cs.pt = pt;
+#pragma unroll
+  for (int i = 0; i < M::NP; i++) L.p[i] = (R)a.params.base[pt * a.params.ps + i * a.params.cs];
+  const R *st = static_cast<const R *>(a.resume.state);
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    L.x[i] = st[i * a.P + pt];
+    if (INTEG == kDopri5) L.kx[i] = st[(N + i) * a.P + pt];
+  }
+  L.h = st[2 * N * a.P + pt];
+  const int64_t steps = a.resume.steps[pt];
+  L.reject = (steps & kResumeReject) != 0;
+  L.steps = steps & ~kResumeReject;
+  cs.t_avg = a.t_avg_per_point ? a.t_avg_per_point[pt] : a.t_avg;
+  L.L = (float)a.dt_renorm / kRenormSplitInit;
+  L.rate_max = initial_renorm_rate(renorm_spread_limit<R>((float)a.rtol), (float)a.dt_renorm);
+#pragma unroll
+  for (int i = 0; i < K; i++) {
+    cs.sum[i] = cs.comp[i] = 0.0;
+    cs.prod[i] = 1.0;
+  }
+  lane_start_tangent(L, a);
+}
+
 // Gram-Schmidt step of one lane: log-norms accumulated in the averaging
 // phase, interval target adapted.  Returns false on a degenerate basis.
 template <class M, int K, class R, int INTEG>
@@ -1162,6 +1192,99 @@ inline BatchArgs with_ctl(const BatchArgs &b, int prec) {
   for (int i = 0; i < b.nseg; i++)
     out.seg[i].ctl = prec == kFP32 ? make_ctl<float>(b.seg[i]) : make_ctl<double>(b.seg[i]);
   return out;
+}
+
+// The transient of one point on one thread: lane_step's steps of the state
+// alone (the same pass -- for FP32 with the tangent row that rides along, zero,
+// so that the states agree bit for bit -- controller, limits and statuses), its
+// end state into a.resume.  A point that ends here writes its outputs.  Cost of
+// the averaging phase: attempts per unit of time so far, times its length.
+template <class M, class R, int INTEG>
+CL_HD void run_transient(const AdaptiveArgs &a, const Ctl &c, int64_t pt) {
+  using C = typename CtlReal<R>::type;
+  constexpr int N = M::N, K = M::N;
+  Lane<M, K, R, INTEG> L;
+  R(&p)[M::NP] = L.p;
+  R(&x)[N] = L.x;
+  R(&kx)[N] = L.kx;
+#pragma unroll
+  for (int i = 0; i < K; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) L.V[i][j] = L.kv[i][j] = R(0);
+#pragma unroll
+  for (int i = 0; i < M::NP; i++) p[i] = (R)a.params.base[pt * a.params.ps + i * a.params.cs];
+#pragma unroll
+  for (int i = 0; i < N; i++) x[i] = (R)a.inits.base[pt * a.inits.ps + i * a.inits.cs];
+  if (INTEG == kDopri5) M::f(x, kx, p);
+  R h = (R)a.h0;
+  C lfac_old = log2_fac_min<C>();
+  bool reject = false;
+  int64_t steps = 0;
+  double t_left = a.t_transient;
+  R t_left_r = time_left_as<R>(t_left);
+  int status = state_inside(x, c.escape) ? -1 : 4;
+  bool done = false;
+  while (status < 0 && !done) {
+    if (steps >= c.max_steps) {
+      status = 3;
+      break;
+    }
+    if (!step_at_least_hmin(h, c)) {
+      status = 2;
+      break;
+    }
+    const bool clamped = h >= t_left_r;
+    const R hs = clamped ? t_left_r : h;
+    R x1[N], V1[K][N], kx1[N], kv1[K][N];
+    steps++;
+    const C err2 = attempt<M, K, R, INTEG>(L, hs, false, ctl_rtol<R>(c), ctl_atol<R>(c), x1, V1,
+                                           kx1, kv1);
+    if (!(err2 <= err2_limit<C>())) {
+      if (!point_finite(p, x)) {
+        status = 1;
+        break;
+      }
+      h = hs / (R)kNonfiniteDiv;
+      reject = true;
+      continue;
+    }
+    R hnew;
+    if (control<R, INTEG>(err2, hs, lfac_old, reject, c, hnew)) {
+#pragma unroll
+      for (int j = 0; j < N; j++) {
+        x[j] = x1[j];
+        if (INTEG == kDopri5) kx[j] = kx1[j];
+      }
+      if (!clamped || hnew < hs) h = hnew;
+      if (!clamped) {
+        t_left -= (double)hs;
+        t_left_r = time_left_as<R>(t_left);
+      }
+      if (!state_inside(x, c.escape)) status = 4;
+      done = clamped;
+    } else {
+      h = hnew;
+    }
+  }
+  if (status >= 0) {
+#pragma unroll
+    for (int i = 0; i < N; i++) a.spectrum.base[pt * a.spectrum.ps + i * a.spectrum.cs] = quiet_nan();
+    if (a.status) a.status[pt] = status;
+    if (a.steps) a.steps[pt] = steps;
+    a.resume.steps[pt] = -1;
+    a.resume.cost[pt] = 0.0;
+    return;
+  }
+  R *st = static_cast<R *>(a.resume.state);
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    st[i * a.P + pt] = x[i];
+    if (INTEG == kDopri5) st[(N + i) * a.P + pt] = kx[i];
+  }
+  st[2 * N * a.P + pt] = h;
+  a.resume.steps[pt] = steps | (reject ? kResumeReject : 0);
+  const double t_avg = a.t_avg_per_point ? a.t_avg_per_point[pt] : a.t_avg;
+  a.resume.cost[pt] = (double)steps * (t_avg / a.t_transient);
 }
 
 // One point start to finish on one thread (the host form of the kernel

@@ -115,6 +115,9 @@ struct chaos_lyap_handle {
   int32_t *order = nullptr;
   void *order_scratch = nullptr;
   int64_t order_cap = 0;
+  // end states of the transients, for sweeps in two launches
+  void *resume = nullptr;
+  int64_t resume_cap = 0;  // points
   // second stream and fork / join events of a batch with both kernel forms
   cudaStream_t aux_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -330,6 +333,7 @@ int chaos_lyap_destroy(chaos_lyap_handle *h) {
   cudaFree(h->queue);
   cudaFree(h->order);
   cudaFree(h->order_scratch);
+  cudaFree(h->resume);
   if (h->aux_stream) {
     cudaStreamSynchronize(h->aux_stream);
     cudaStreamDestroy(h->aux_stream);
@@ -357,6 +361,49 @@ static int ensure_order(chaos_lyap_handle *h, int64_t P) {
     return fail(CHAOS_LYAP_ENOMEM, "cudaMalloc(order): %s", cudaGetErrorString(e));
   }
   h->order_cap = P;
+  return CHAOS_LYAP_OK;
+}
+
+// A persistent one-lane sweep runs as two launches -- all transients, then the
+// averaging phases, those expected to take longest first -- when its points
+// are more than the GPU holds at once (otherwise every point starts at once and
+// the order cannot matter; just above one wave the run is its longest points
+// either way) but few enough waves that the end of the run, where lanes wait
+// for the longest points started last, is a sizeable part of it.  Needs a
+// transient (it is what predicts the cost); the buffers, 48-76 bytes per point,
+// are kept by the handle.  One launch -> two, B200: 256^2 Lorenz points in FP64
+// (1.7 waves) 245 -> 195 ms; FP32 Lorenz, 152k points (2 waves) 62 -> 47 ms,
+// 300k 103 -> 85 ms, 1024^2 (14 waves) 309 -> 275 ms; FP32 Rossler, whose
+// longest points take twice the mean, 152k points 82 -> 77 ms; at 1.1 waves of
+// it 55 -> 52 ms.
+constexpr double kTwoPhaseMinWaves = 1.5;
+constexpr int64_t kTwoPhaseMaxWaves = 32;
+
+// Buffers of a two-launch sweep of P points; *ready false during a stream
+// capture (a replay must not depend on buffers that a later run of the handle
+// may grow) or when memory is short: the sweep then runs as one launch.
+static int ensure_resume(chaos_lyap_handle *h, int64_t P, cudaStream_t s, bool *ready) {
+  *ready = false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &cap);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
+  if (cap != cudaStreamCaptureStatusNone) return CHAOS_LYAP_OK;
+  if (P > h->resume_cap) {
+    DeviceGuard g(h->d.device);
+    cudaFree(h->resume);
+    h->resume = nullptr;
+    h->resume_cap = 0;
+    const int prec = h->d.precision == CHAOS_PREC_FP32 ? chaos::kFP32 : chaos::kFP64;
+    if (cudaMalloc(&h->resume, (chaos::resume_state_bytes(h->model->dim, prec) + 16) * P) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      h->resume = nullptr;
+      return CHAOS_LYAP_OK;
+    }
+    h->resume_cap = P;
+  }
+  *ready = ensure_order(h, P) == CHAOS_LYAP_OK;
+  if (!*ready) cudaGetLastError();
   return CHAOS_LYAP_OK;
 }
 
@@ -420,6 +467,28 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
       if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(queue)");
       a.queue = h->queue;
       a.queue_stride = chaos::queue_stride_for(P);
+      bool two_phase = false;
+      if (!split && m->dim <= 4 && a.t_transient > 0) {
+        const int64_t lanes = chaos::adaptive_resident(m->id, integ, prec, block, variant);
+        if (P >= (int64_t)(kTwoPhaseMinWaves * lanes) && P <= kTwoPhaseMaxWaves * lanes &&
+            (rc = ensure_resume(h, P, s, &two_phase)))
+          return rc;
+      }
+      if (two_phase) {
+        a.order = h->order;
+        a.resume.cost = static_cast<double *>(h->resume);
+        a.resume.steps = reinterpret_cast<int64_t *>(a.resume.cost + P);
+        a.resume.state = a.resume.steps + P;
+        rc = chaos::launch_adaptive_two_phase(m->id, integ, prec, a, block, variant,
+                                              h->order_scratch, s);
+        if (rc && rc != chaos::kErrUnsupported) return cuda_fail((cudaError_t)rc, "kernel launch");
+        if (!rc) {
+          h->last_stream = s;
+          return CHAOS_LYAP_OK;
+        }
+        a.resume = chaos::Resume{};
+        a.order = nullptr;
+      }
       if (a.t_avg_per_point && m->dim <= 4) {  // longest averaging time first
         if ((rc = ensure_order(h, P))) return rc;
         rc = chaos::launch_order_longest_first(a.t_avg_per_point, P, h->order, h->order_scratch, s);
@@ -429,7 +498,7 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
     }
     if (m->dim > 4) rc = chaos::launch_l96_warp(integ, prec, a, 0, s);
     else if (split) rc = chaos::launch_split(m->id, integ, prec, a, block, variant, s);
-    else rc = chaos::launch_adaptive(m->id, integ, prec, a, block, 0, variant, s);
+    else rc = chaos::launch_adaptive(m->id, integ, prec, a, block, variant, s);
   }
   if (rc == chaos::kErrUnsupported)
     return fail(CHAOS_LYAP_EUNSUPPORTED, "no kernel for model %s with this integrator/precision/k",

@@ -50,6 +50,19 @@ struct Ctl {
   double escape;
 };
 
+// What the transient of a point leaves behind for its averaging phase when the
+// two run as separate launches (adaptive.cu: transient_kernel).  state holds
+// 2 N + 1 values of the step's precision per point, component by component
+// (x, its derivative, the step proposal: value c of point pt at state[c * P +
+// pt]).
+struct Resume {
+  void *state;
+  int64_t *steps;  // attempted steps; bit 62: the last attempt was rejected;
+                   // negative: the point ended in its transient
+  double *cost;    // expected cost of the averaging phase (attempts)
+};
+constexpr int64_t kResumeReject = 1LL << 62;
+
 // Adaptive forms (DVERK 6(5) or Dopri5; FP64 or FP32 state and tangent; FP64
 // Gram-Schmidt and compensated log-norm sums).
 struct AdaptiveArgs {
@@ -69,6 +82,7 @@ struct AdaptiveArgs {
   unsigned long long *queue;  // nullable unless the launch is persistent
   uint64_t queue_stride;      // coprime to P: hand-out order q -> q * stride mod P
   const int32_t *order;       // nullable: hand-out order q -> order[q] (overrides the stride)
+  Resume resume;              // state null: each point runs from its initial state
   Ctl ctl;                    // set by the launchers from the fields above
 };
 
@@ -99,7 +113,18 @@ constexpr int kErrUnsupported = -1;
 int launch_compat(int model, const CompatArgs &a, int block, cudaStream_t s);
 // variant: 0 = 128-register build, 1 = 96-register build (FP32 only)
 int launch_adaptive(int model, int integrator, int precision, const AdaptiveArgs &a, int block,
-                    int persistent_blocks, int variant, cudaStream_t s);
+                    int variant, cudaStream_t s);
+// Two launches: the transients of all points, then their averaging phases,
+// longest expected first (a.order must point to P entries, order_scratch to
+// kOrderScratchBytes, a.resume to buffers of P points).
+int launch_adaptive_two_phase(int model, int integrator, int precision, const AdaptiveArgs &a,
+                              int block, int variant, void *order_scratch, cudaStream_t s);
+// Points a persistent launch of this form holds at once on the current device.
+int64_t adaptive_resident(int model, int integrator, int precision, int block, int variant);
+// Bytes of Resume::state per point.
+inline int64_t resume_state_bytes(int dim, int precision) {
+  return (2 * dim + 1) * (precision == kFP32 ? 4 : 8);
+}
 int launch_l96_warp(int integrator, int precision, const AdaptiveArgs &a, int warps_per_block,
                     cudaStream_t s);
 
