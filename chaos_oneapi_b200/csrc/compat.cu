@@ -1,7 +1,7 @@
 // Reference-exact FP64 sweep ("compat" precision).
 //
-// One thread per parameter point, the model inlined as a template parameter,
-// state / tangent vectors / DVERK stages in registers (the reference keeps
+// One thread per parameter point (few points: one lane per row of a point, see
+// compat_rows_kernel), the model inlined as a template parameter, state / tangent vectors / DVERK stages in registers (the reference keeps
 // them in per-work-item global scratch, tasklyapunov.cpp:104-176).  The
 // arithmetic follows the reference operation by operation so that, compiled
 // with -fmad=false (no FMA contraction), trajectories agree bit for bit with
@@ -356,8 +356,215 @@ __global__ void __launch_bounds__(128) compat_kernel(const CompatArgs a) {
   if (a.status) a.status[pt] = finite ? 0 : 1;
 }
 
+// ------------------------------------------------- one row per lane
+// Flows of dimension <= 4 with few points: a point takes a group of G lanes,
+// lane 0 the state (and the lanes past the last vector copies of it), lane 1 + i
+// tangent vector / perturbed trajectory / column i.  The rows of a step are
+// independent given the state at its start, so a step's chain is one DVERK row
+// instead of 1 + k, and Gram-Schmidt's divisions, square roots and logarithms
+// run beside each other.  Every row goes through the operations of the
+// one-thread form in their order (no multiply-add is contracted here): the same
+// bits.  The price is the state-only phase, which every lane repeats, and a
+// right-hand side evaluated for both kinds of row; see kMaxLanePointsPerSm.
+template <int N> struct Rows {
+  int i;          // vector index, < 0: the state
+  int base;       // the group's first lane
+  unsigned mask;  // the group's lanes
+  __device__ __forceinline__ void from(int lane, const double (&v)[N], double (&out)[N]) const {
+#pragma unroll
+    for (int q = 0; q < N; q++) out[q] = __shfl_sync(mask, v[q], base + lane);
+  }
+};
+
+// A row's derivative: f for the state rows, J(X) v (or column J(X) q) for the
+// others, both evaluated and one selected (a branch would run one after the
+// other).
+template <class M, bool QR> struct DRow {
+  const double *p, *X;
+  bool vec;
+  __device__ __forceinline__ void operator()(const double *y, double *dy) const {
+    double f[M::N], g[M::N];
+    M::f(y, f, p);
+    if (QR) M::jq_col(y, g, p, X);
+    else M::jv(y, g, p, X);
+#pragma unroll
+    for (int q = 0; q < M::N; q++) dy[q] = vec ? g[q] : f[q];
+  }
+};
+
+// ort_vecs over the group: round j takes the finished vector j from its lane.
+template <int N, int K>
+__device__ __forceinline__ void ort_rows(double (&v)[N], const Rows<N> &g) {
+  double proj[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) proj[q] = 0;
+#pragma unroll
+  for (int j = 0; j + 1 < K; j++) {
+    double vj[N];
+    g.from(1 + j, v, vj);
+    if (g.i > j) {
+      const double c = dot_seq<N>(vj, v) / dot_seq<N>(vj, vj);
+#pragma unroll
+      for (int q = 0; q < N; q++) proj[q] += c * vj[q];
+      if (g.i == j + 1) {
+#pragma unroll
+        for (int q = 0; q < N; q++) v[q] -= proj[q];
+      }
+    }
+  }
+}
+template <int N> __device__ __forceinline__ void normalize_row(double (&v)[N], double eps) {
+  const double nr = sqrt(dot_seq<N>(v, v));
+#pragma unroll
+  for (int q = 0; q < N; q++) v[q] = (v[q] / nr) * eps;
+}
+
+// point_var / point_fd on a group; y: this lane's row.  X: the state.
+template <class M, int K, bool FD>
+__device__ __forceinline__ void rows_var_fd(const CompatArgs &a, const double *p,
+                                            double (&X)[M::N], double (&y)[M::N], double &lyap,
+                                            const Rows<M::N> &g) {
+  constexpr int N = M::N;
+  const double h = a.step;
+  const bool vec = g.i >= 0;
+  DState<M> fs{p};
+  for (double t = 0; t < a.t_skip; t += h) dverk<N>(X, fs, h);
+#pragma unroll
+  for (int q = 0; q < N; q++) y[q] = FD || !vec ? X[q] : 0.;
+#pragma unroll
+  for (int q = 0; q < N; q++)
+    if (q == g.i) y[q] += a.eps;
+  auto step = [&]() {
+    if (FD) dverk<N>(y, fs, h);
+    else dverk<N>(y, DRow<M, false>{p, X, vec}, h);
+    g.from(0, y, X);
+  };
+  auto offset = [&](double sign) {  // FD: rows relative to the state, and back
+    if (FD && vec) {
+#pragma unroll
+      for (int q = 0; q < N; q++) y[q] = sign < 0 ? y[q] - X[q] : y[q] + X[q];
+    }
+  };
+  for (double t = 0; t < a.t_skip_clp; t += h) {
+    step();
+    offset(-1);
+    ort_rows<N, K>(y, g);
+    if (vec) normalize_row<N>(y, a.eps);
+    offset(1);
+  }
+  int32_t skip = 0;
+  for (double t = 0; t < a.calc_time; t += h) {
+    skip++;
+    step();
+    if (skip == a.add_skip) {
+      offset(-1);
+      ort_rows<N, K>(y, g);
+      if (vec) {
+        lyap += log(sqrt(dot_seq<N>(y, y)) / a.eps);
+        normalize_row<N>(y, a.eps);
+      }
+      offset(1);
+      skip = 0;
+    }
+  }
+  lyap = lyap / a.calc_time;
+}
+
+// point_qr on a group.  A column's step needs the state after the state's step;
+// the state's lane runs one step ahead, so that both advance together.
+template <class M>
+__device__ __forceinline__ void rows_qr(const CompatArgs &a, const double *p, double (&X)[M::N],
+                                        double (&y)[M::N], double &lyap, const Rows<M::N> &g) {
+  constexpr int N = M::N;
+  const double h = a.step, end = a.t_skip + a.calc_time;
+  const bool vec = g.i >= 0;
+  DState<M> fs{p};
+  for (double t = 0; t < a.t_skip; t += h) dverk<N>(X, fs, h);
+#pragma unroll
+  for (int q = 0; q < N; q++) y[q] = q == g.i ? 1. : 0.;
+  double ahead[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) ahead[q] = X[q];
+  if (a.t_skip < end) dverk<N>(ahead, fs, h);
+  for (double t = a.t_skip; t < end; t += h) {
+#pragma unroll
+    for (int q = 0; q < N; q++) X[q] = ahead[q];
+    if (!vec) {
+#pragma unroll
+      for (int q = 0; q < N; q++) y[q] = X[q];
+    }
+    dverk<N>(y, DRow<M, true>{p, X, vec}, h);
+    g.from(0, y, ahead);
+    double A[N];
+#pragma unroll
+    for (int q = 0; q < N; q++) A[q] = y[q];
+    ort_rows<N, N>(y, g);
+    if (vec) {
+      normalize_row<N>(y, 1);
+      lyap += log(fabs(dot_seq<N>(y, A)));
+    }
+  }
+  lyap = lyap / a.calc_time;
+}
+
+template <class M, int K, int G>
+__global__ void __launch_bounds__(32) compat_rows_kernel(const CompatArgs a) {
+  constexpr int N = M::N;
+  const int lane = threadIdx.x & 31, r = lane % G;
+  const int64_t pt = (int64_t)blockIdx.x * (32 / G) + lane / G;
+  if (pt >= a.P) return;  // whole groups
+  const Rows<N> g{r >= 1 && r <= K ? r - 1 : -1, lane - r,
+                  (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << (lane - r)};
+  double p[M::NP], X[N], y[N], lyap = 0.;
+#pragma unroll
+  for (int i = 0; i < M::NP; i++) p[i] = a.params.base[pt * a.params.ps + i * a.params.cs];
+#pragma unroll
+  for (int i = 0; i < N; i++) X[i] = a.inits.base[pt * a.inits.ps + i * a.inits.cs];
+  __syncwarp(g.mask);  // every lane of the group has read the state that lane 0 replaces
+  double *out = a.lyap.base + pt * a.lyap.ps + g.i * a.lyap.cs;
+  if (a.accumulate && g.i >= 0) lyap = *out;
+  if (a.method == 2) {
+    if constexpr (K == N) rows_qr<M>(a, p, X, y, lyap, g);
+  } else {
+    if (a.method == 1) rows_var_fd<M, K, false>(a, p, X, y, lyap, g);
+    else rows_var_fd<M, K, true>(a, p, X, y, lyap, g);
+    if (a.close && g.i >= 0) {
+#pragma unroll
+      for (int q = 0; q < N; q++) a.close[(pt * K + g.i) * N + q] = y[q];
+    }
+  }
+  if (g.i >= 0) *out = lyap;
+  if (r == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i++) a.inits.base[pt * a.inits.ps + i * a.inits.cs] = X[i];
+  }
+  const bool finite = __all_sync(g.mask, g.i < 0 || isfinite(lyap));
+  if (a.status && r == 0) a.status[pt] = finite ? 0 : 1;
+}
+
+// Up to this many points per SM a group of lanes per point is faster than a
+// thread.  One thread per point is one row's latency times 1 + k until its
+// threads fill the schedulers (16,384 points: one warp each); the groups are
+// bound by the FP64 pipe from about 30 points per SM on.  800 steps, k = 3, one
+// thread / group: Shimizu FD 1,024 points 967 / 328 us, 7,680 points 973 / 523,
+// 12,288 points 975 / 737, 16,384 points 976 / 958, 25,600 points 1464 / 1384;
+// Lorenz QR 1,024 points 1386 / 654 us, 12,288 points 1390 / 1168, 16,384 points
+// 1391 / 1474; Lorenz VAR 12,288 points 1028 / 863, 16,384 points 1028 / 1120.
+constexpr int64_t kMaxLanePointsPerSm = 88;
+
 template <class M, int KT>
 int launch_one(const CompatArgs &a, int block, cudaStream_t s) {
+  if constexpr (KT > 0 && !IsMap<M>::value) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (a.P <= kMaxLanePointsPerSm * sms && (a.method != 2 || KT == M::N)) {
+      constexpr int G = KT + 1 <= 2 ? 2 : KT + 1 <= 4 ? 4 : 8;
+      const int64_t grid = (a.P + 32 / G - 1) / (32 / G);
+      compat_rows_kernel<M, KT, G><<<(unsigned)grid, 32, 0, s>>>(a);
+      return (int)cudaGetLastError();
+    }
+  }
   const int64_t grid = (a.P + block - 1) / block;
   compat_kernel<M, KT><<<(unsigned)grid, block, 0, s>>>(a);
   return (int)cudaGetLastError();
