@@ -17,8 +17,9 @@
 // J(x) v at the step's start costs one stencil pass with the stage-0
 // Jacobian coefficients the state pass computes anyway (the same floats an
 // FSAL copy would hold), and leaving them out halves the shared memory per
-// point, so twice as many points fit on an SM.  The FP64 QR widens the
-// vectors in place over both halves (k x 40 doubles).
+// point, so twice as many points fit on an SM.  Gram-Schmidt works on
+// FP64 copies in registers, two lanes per vector, and keeps the finished ones
+// over both halves (k x 40 doubles); see mgs_qr.
 //
 // The phase and renormalisation logic follows adaptive.cuh (transient /
 // alignment / averaging with clamped landings, the renormalisation interval
@@ -39,7 +40,6 @@ constexpr int N = 40;        // model dimension
 constexpr int G = 4;         // vectors processed at once per warp (lane groups)
 constexpr int C = 5;         // components per lane
 constexpr int WARPS = 4;     // warps (points) per block
-constexpr int PV = 4;        // Gram-Schmidt: later vectors per lane group per projection round
 constexpr unsigned FULL = 0xffffffffu;
 
 struct DPc {  // Dormand-Prince 5(4), cuda/tools/dopri.dp.cpp:14-44
@@ -90,6 +90,23 @@ struct Jc {
   float A[C], B[C];
 };
 
+// a b + c d and the longer sums of the passes below, left to right, with their
+// multiply-adds explicit: the compiler may fuse either product, and a sweep's
+// step sequence must not depend on its choice.
+__device__ __forceinline__ float lin(float a, float b, float c, float d) {
+  return fmaf(a, b, __fmul_rn(c, d));
+}
+__device__ __forceinline__ float lin_on(float acc) { return acc; }
+template <class... R>
+__device__ __forceinline__ float lin_on(float acc, float c, float k, R... r) {
+  return lin_on(fmaf(c, k, acc), r...);
+}
+template <class... R>
+__device__ __forceinline__ float lin(float c1, float k1, float c2, float k2, float c3, float k3,
+                                     R... r) {
+  return lin_on(lin(c1, k1, c2, k2), c3, k3, r...);
+}
+
 __device__ __forceinline__ void rhs_state(const float (&x)[C], float (&dx)[C], Jc &jc, float F,
                                           float gam, int left, int right) {
   const Win e = window(x, neighbours(x, left, right));
@@ -97,7 +114,7 @@ __device__ __forceinline__ void rhs_state(const float (&x)[C], float (&dx)[C], J
   for (int j = 0; j < C; j++) {
     jc.A[j] = e.at(j - 1);
     jc.B[j] = e.at(j + 1) - e.at(j - 2);
-    dx[j] = jc.B[j] * jc.A[j] - gam * e.at(j) + F;
+    dx[j] = lin(jc.B[j], jc.A[j], -gam, e.at(j)) + F;
   }
 }
 
@@ -106,13 +123,14 @@ __device__ __forceinline__ void rhs_tangent(const float (&v)[C], float (&dv)[C],
   const Win e = window(v, neighbours(v, left, right));
 #pragma unroll
   for (int j = 0; j < C; j++)
-    dv[j] = (e.at(j + 1) - e.at(j - 2)) * jc.A[j] + jc.B[j] * e.at(j - 1) - gam * e.at(j);
+    dv[j] = fmaf(-gam, e.at(j), lin(e.at(j + 1) - e.at(j - 2), jc.A[j], jc.B[j], e.at(j - 1)));
 }
 
-__device__ __forceinline__ float err_term(float y0, float y1, float e, float rtol, float atol) {
+__device__ __forceinline__ float err_term(float y0, float y1, float e, float rtol, float atol,
+                                          float acc) {
   const float m = fmaxf(fabsf(y0), fabsf(y1));
   const float r = __fdividef(e, fmaf(rtol, m, atol));
-  return r * r;
+  return fmaf(r, r, acc);
 }
 
 // One Dopri5 pass over the lane's 5 components.  rhs(s, arg, out) evaluates
@@ -124,39 +142,40 @@ __device__ __forceinline__ void dopri_pass(const float (&y)[C], const float (&k1
   using T = DPc;
   float k2[C], k3[C], k4[C], k5[C], arg[C], e[C];
 #pragma unroll
-  for (int j = 0; j < C; j++) arg[j] = y[j] + h * (T::a21 * k1[j]);
+  for (int j = 0; j < C; j++) arg[j] = fmaf(h, __fmul_rn(T::a21, k1[j]), y[j]);
   rhs(1, arg, k2);
 #pragma unroll
-  for (int j = 0; j < C; j++) arg[j] = y[j] + h * (T::a31 * k1[j] + T::a32 * k2[j]);
+  for (int j = 0; j < C; j++) arg[j] = fmaf(h, lin(T::a31, k1[j], T::a32, k2[j]), y[j]);
   rhs(2, arg, k3);
 #pragma unroll
-  for (int j = 0; j < C; j++) arg[j] = y[j] + h * (T::a41 * k1[j] + T::a42 * k2[j] + T::a43 * k3[j]);
+  for (int j = 0; j < C; j++)
+    arg[j] = fmaf(h, lin(T::a41, k1[j], T::a42, k2[j], T::a43, k3[j]), y[j]);
   rhs(3, arg, k4);
 #pragma unroll
   for (int j = 0; j < C; j++)
-    arg[j] = y[j] + h * (T::a51 * k1[j] + T::a52 * k2[j] + T::a53 * k3[j] + T::a54 * k4[j]);
+    arg[j] = fmaf(h, lin(T::a51, k1[j], T::a52, k2[j], T::a53, k3[j], T::a54, k4[j]), y[j]);
   rhs(4, arg, k5);
 #pragma unroll
   for (int j = 0; j < C; j++) {
-    arg[j] = y[j] + h * (T::a61 * k1[j] + T::a62 * k2[j] + T::a63 * k3[j] + T::a64 * k4[j] +
-                         T::a65 * k5[j]);
-    e[j] = T::e1 * k1[j] + T::e3 * k3[j] + T::e4 * k4[j] + T::e5 * k5[j];
-    y1[j] = T::b1 * k1[j] + T::b3 * k3[j] + T::b4 * k4[j] + T::b5 * k5[j];
+    arg[j] = fmaf(h, lin(T::a61, k1[j], T::a62, k2[j], T::a63, k3[j], T::a64, k4[j], T::a65, k5[j]),
+                  y[j]);
+    e[j] = lin(T::e1, k1[j], T::e3, k3[j], T::e4, k4[j], T::e5, k5[j]);
+    y1[j] = lin(T::b1, k1[j], T::b3, k3[j], T::b4, k4[j], T::b5, k5[j]);
   }
   {
     float k6[C];
     rhs(5, arg, k6);
 #pragma unroll
     for (int j = 0; j < C; j++) {
-      y1[j] = y[j] + h * (y1[j] + T::b6 * k6[j]);
-      e[j] += T::e6 * k6[j];
+      y1[j] = fmaf(h, fmaf(T::b6, k6[j], y1[j]), y[j]);
+      e[j] = fmaf(T::e6, k6[j], e[j]);
     }
   }
   rhs(6, y1, k7);
 #pragma unroll
   for (int j = 0; j < C; j++) {
-    e[j] += T::e7 * k7[j];
-    err2 += err_term(y[j], y1[j], h * e[j], rtol, atol);
+    e[j] = fmaf(T::e7, k7[j], e[j]);
+    err2 = err_term(y[j], y1[j], h * e[j], rtol, atol, err2);
   }
 }
 
@@ -165,12 +184,6 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
   return v;
 }
-__device__ __forceinline__ double group_sum(double v) {  // over the 8 lanes of a group
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  return v;
-}
-
 enum Phase : int { kTransient = 0, kAlign = 1, kAverage = 2 };
 
 struct Warp {
@@ -197,128 +210,167 @@ __device__ __forceinline__ void flush_logs(Warp &w) {
   }
 }
 
-// In-place conversions between the k x 40 FP32 vectors and their FP64 copy
-// W, which covers the warp's whole 2 x k x 40-float area (base).  The FP32
-// vectors are in its lower half (src_upper false) or upper half.  Chunks of
-// 32 elements, each read whole (__syncwarp) before it is written, in the
-// order that never overwrites an element not yet read: widening from the
-// lower half runs downwards (double i covers floats 2i, 2i + 1 >= i),
-// widening from the upper half and narrowing into the lower half run upwards.
-__device__ void widen(const float *src, double *W, int n, int lane, bool src_upper) {
-  const int nch = (n + 31) / 32;
-  for (int c = 0; c < nch; c++) {
-    const int idx = 32 * (src_upper ? c : nch - 1 - c) + lane;
-    const float f = idx < n ? src[idx] : 0.f;
-    __syncwarp();
-    if (idx < n) W[idx] = (double)f;
-    __syncwarp();
-  }
+// Gram-Schmidt layout.  Two lanes hold one vector in registers, 20 components
+// each, so a warp orthogonalises a block of 16 vectors at once; the finished
+// vectors lie in shared memory in FP64.  The 40 components are eight runs of
+// five; lane 0 of a pair takes runs 0, 4, 2, 6, lane 1 runs 1, 5, 3, 7, each
+// lane's 20 contiguous in shared memory (gs_pos).  A dot product is a chain of
+// five multiply-adds per run, the runs added as ((0 + 4) + (2 + 6)) + ((1 + 5) +
+// (3 + 7)): two additions in the lane and one exchange in the pair.  (With one
+// run per lane, the layout of the steps, the same sum was three shuffle levels
+// per dot product, and each vector was read and rewritten in shared memory for
+// every earlier one.)
+constexpr int kPairVecs = 16;
+__device__ __forceinline__ int gs_run(int half, int i) {  // run i of a lane's four
+  return half + ((i & 1) << 2) + (i & 2);
 }
-__device__ void narrow(const double *W, float *dst, int n, int lane) {
-  const int nch = (n + 31) / 32;
-  for (int c = 0; c < nch; c++) {
-    const int idx = 32 * c + lane;
-    const double d = idx < n ? W[idx] : 0.0;
-    __syncwarp();
-    if (idx < n) dst[idx] = (float)d;
-    __syncwarp();
+__device__ __forceinline__ int gs_pos(int run) {  // first double of a run in a stored vector
+  return (run & 1) * 20 + (((run >> 2) & 1) + (run & 2)) * 5;
+}
+
+// The lane's half of a dot product with the stored half vector q (16-byte
+// aligned; both lanes of every pair read the same two addresses: broadcasts).
+__device__ __forceinline__ double pair_sum(const double (&p)[4]) {
+  const double h = (p[0] + p[1]) + (p[2] + p[3]);
+  return h + __shfl_xor_sync(FULL, h, 1);
+}
+__device__ __forceinline__ double dot_stored(const double2 *q, const double (&w)[20]) {
+  double p[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < 10; i++) {
+    const double2 t = q[i];
+    p[(2 * i) / 5] = fma(t.x, w[2 * i], p[(2 * i) / 5]);
+    p[(2 * i + 1) / 5] = fma(t.y, w[2 * i + 1], p[(2 * i + 1) / 5]);
+  }
+  return pair_sum(p);
+}
+__device__ __forceinline__ double dot_self(const double (&w)[20]) {
+  double p[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < 20; i++) p[i / 5] = fma(w[i], w[i], p[i / 5]);
+  return pair_sum(p);
+}
+__device__ __forceinline__ void subtract_stored(const double2 *q, double c, double (&w)[20]) {
+#pragma unroll
+  for (int i = 0; i < 10; i++) {
+    const double2 t = q[i];
+    w[2 * i] = fma(-c, t.x, w[2 * i]);
+    w[2 * i + 1] = fma(-c, t.y, w[2 * i + 1]);
   }
 }
 
 // Modified Gram-Schmidt in FP64 on the k vectors of V (k x 40, FP32, in the
-// lower or upper half of the warp's area `base`), through the FP64 work area
-// W = base (k x 40 doubles); the orthonormal vectors end in the lower half.
-// Returns max |v_q|^2 / r_q^2 (the cancellation factor), the smallest r_q in
-// rmin, and multiplies r_q into the lane that owns exponent q.
-__device__ double mgs_qr(Warp &w, const float *V, float *base, int k, int g, int li, int lane,
-                         bool accumulate, bool &ok, double &rmin) {
+// lower or upper half of the warp's area `base`, 2 k x 40 floats); the
+// orthonormal vectors end in the lower half.
+//
+// Left-looking: a block of 16 vectors is loaded into registers, the finished
+// vectors before it are projected out one by one, then the block's own, each
+// normalised and stored as its turn comes.  Every vector meets its predecessors
+// in the same order as in the right-looking form, with the same operations.
+// The area holds the finished vectors in FP64 (vector q over floats 80 q ..
+// 80 q + 79) while the later ones wait in the upper half (vector j at floats
+// 40 k + 40 j): storing the vectors of block b, the last at 80 (16 b + 15) + 79,
+// never reaches the first one not yet loaded, at 40 k + 640 (b + 1), since
+// that one exists only if 16 (b + 1) < k.
+// A pass of 40 vectors is a chain of 40 normalisations (dot product, reciprocal
+// root, store, dot product) and about 6,000 FP64 instructions; beside three
+// other warps on the scheduler it takes 91,000 cycles (right-looking, with one
+// run per lane: 135,000, 71 % of the sweep's time).  64^2 points, T 5 + 50:
+// 135.8 -> 115.9 ms.
+struct GsResult {
+  double cancel;  // max |v_q|^2 / r_q^2, the cancellation factor
+  double rmin;    // the smallest r_q
+  double r[2];    // r_q of the exponents this lane owns (lane, lane + 32); else 1
+  bool ok;
+};
+// (not inlined: its registers are the vectors', the step's are saved around the
+// call, once per pass)
+__device__ __noinline__ GsResult mgs_qr(const float *V, float *base, int k, int lane) {
   double *W = reinterpret_cast<double *>(base);
-  widen(V, W, k * N, lane, V != base);
-  // squared norms before orthogonalisation: vector q's in lane q % 32, slot q / 32
-  double nb[2] = {0.0, 0.0};
-  for (int r = 0; r < (k + G - 1) / G; r++) {
-    const int vec = r * G + g;
-    double b = 0;
+  float *U = base + k * N;
+  if (V == base) {  // to the upper half
+    for (int i = lane; i < k * N / 4; i += 32)
+      reinterpret_cast<float4 *>(U)[i] = reinterpret_cast<const float4 *>(V)[i];
+    __syncwarp();
+  }
+  const int pair = lane >> 1, half = lane & 1;
+  double cancel = 1.0, rmin = 1e300;
+  GsResult res;
+  res.r[0] = res.r[1] = 1.0;
+  res.ok = true;
+  for (int v0 = 0; v0 < k; v0 += kPairVecs) {
+    const int vec = v0 + pair;
+    double x[20];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < C; j++)
+        x[i * C + j] = vec < k ? (double)U[vec * N + gs_run(half, i) * C + j] : 0.0;
+    const double nb = dot_self(x);  // squared norm before the projections
+    __syncwarp();                   // the whole block is in registers
+    for (int q = 0; q < v0; q++) {
+      const double2 *wq = reinterpret_cast<const double2 *>(W + q * N + half * 20);
+      const double c = dot_stored(wq, x);
+      subtract_stored(wq, c, x);
+    }
+    const int nv = min(kPairVecs, k - v0);
+    double s = 1.0, r = 1.0;
+    for (int i = 0; i < nv; i++) {
+      const double t = dot_self(x);  // every pair's; vector i's counts
+      double2 *wq = reinterpret_cast<double2 *>(W + (v0 + i) * N + half * 20);
+      if (pair == i) {
+        s = t;
+        const double inv = rsqrt(t);
+        r = t * inv;
+#pragma unroll
+        for (int j = 0; j < 20; j++) x[j] *= inv;
+#pragma unroll
+        for (int j = 0; j < 10; j++) wq[j] = make_double2(x[2 * j], x[2 * j + 1]);
+      }
+      __syncwarp();
+      if (i + 1 < nv) {
+        const double c = dot_stored(wq, x);
+        if (pair > i) subtract_stored(wq, c, x);
+      }
+    }
+    const bool mine = vec < k;
+    res.ok = __all_sync(FULL, !mine || ((r > 0.0) && (r < 1e300))) && res.ok;
+    if (mine) {
+      rmin = fmin(rmin, r);
+      // norm before any projection vs r (the first vector has none)
+      if (vec > 0) cancel = fmax(cancel, nb / s);
+    }
+    // the norms to the lanes that own their exponents: q in lane q % 32, slot q / 32
+    const double rq = __shfl_sync(FULL, r, 2 * (lane & (kPairVecs - 1)));
+    const int q = v0 + (lane & (kPairVecs - 1));
+    if (q < k && (q & 31) == lane) {
+      if (q >> 5) res.r[1] = rq;
+      else res.r[0] = rq;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    cancel = fmax(cancel, __shfl_xor_sync(FULL, cancel, o));
+    rmin = fmin(rmin, __shfl_xor_sync(FULL, rmin, o));
+  }
+  // FP64 -> FP32 into the lower half, four vectors at a time, each chunk read
+  // whole before it is written: vector q's floats end below 160 (q + 1) bytes,
+  // its unread doubles start at 320 q.
+  for (int v0 = 0; v0 < k; v0 += G) {
+    const int vec = v0 + (lane >> 3), run = lane & 7;
+    double d[C];
+#pragma unroll
+    for (int j = 0; j < C; j++) d[j] = vec < k ? W[vec * N + gs_pos(run) + j] : 0.0;
+    __syncwarp();
     if (vec < k) {
 #pragma unroll
-      for (int j = 0; j < C; j++) {
-        const double vb = W[vec * N + li * C + j];
-        b = fma(vb, vb, b);
-      }
-    }
-    b = group_sum(b);
-#pragma unroll
-    for (int gg = 0; gg < G; gg++) {
-      const double bv = __shfl_sync(FULL, b, gg * 8);
-      const int q = r * G + gg;
-      if (q < k && (q & 31) == lane) nb[q >> 5] = bv;
-    }
-  }
-  __syncwarp();
-  double cancel = 1.0;
-  ok = true;
-  rmin = 1e300;
-  for (int q = 0; q < k; q++) {
-    double wq[C];
-#pragma unroll
-    for (int j = 0; j < C; j++) wq[j] = W[q * N + li * C + j];
-    double s = 0;
-#pragma unroll
-    for (int j = 0; j < C; j++) s = fma(wq[j], wq[j], s);
-    s = group_sum(s);
-    const double inv = rsqrt(s);
-    const double r = s * inv;
-    ok = ok && (r > 0.0) && (r < 1e300);
-    rmin = fmin(rmin, r);
-#pragma unroll
-    for (int j = 0; j < C; j++) wq[j] *= inv;
-    __syncwarp();
-    if (g == 0) {
-#pragma unroll
-      for (int j = 0; j < C; j++) W[q * N + li * C + j] = wq[j];
-    }
-    // projections of the later vectors, G x PV at a time: each group takes
-    // PV vectors per round, whose dot products and group sums are
-    // independent chains that overlap (a round is latency-bound: a 5-term
-    // FP64 dot product and three shuffle levels)
-    for (int j0 = q + 1; j0 < k; j0 += G * PV) {
-      double wj[PV][C], c[PV];
-#pragma unroll
-      for (int u = 0; u < PV; u++) {
-        const int vj = j0 + u * G + g;
-        const bool valid = vj < k;
-#pragma unroll
-        for (int j = 0; j < C; j++) wj[u][j] = valid ? W[vj * N + li * C + j] : 0.0;
-        c[u] = 0.0;
-#pragma unroll
-        for (int j = 0; j < C; j++) c[u] = fma(wq[j], wj[u][j], c[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < PV; u++) c[u] = group_sum(c[u]);
-#pragma unroll
-      for (int u = 0; u < PV; u++) {
-        const int vj = j0 + u * G + g;
-        if (vj < k)
-#pragma unroll
-          for (int j = 0; j < C; j++) W[vj * N + li * C + j] = fma(-c[u], wq[j], wj[u][j]);
-      }
+      for (int j = 0; j < C; j++) base[vec * N + run * C + j] = (float)d[j];
     }
     __syncwarp();
-    if (ok) {
-      // cancellation: norm before any projection vs r (the first vector has none)
-      if (q > 0) {
-        const double b = __shfl_sync(FULL, (q >> 5) ? nb[1] : nb[0], q & 31);
-        cancel = fmax(cancel, b / s);
-      }
-      if (accumulate && (q & 31) == lane) {
-        const int slot = q >> 5;
-        w.prod[slot] *= r;
-      }
-    }
   }
-  __syncwarp();
-  narrow(W, base, k * N, lane);
-  return cancel;
+  res.cancel = cancel;
+  res.rmin = rmin;
+  return res;
 }
 
 __device__ void finish(Warp &w, const AdaptiveArgs &a, int k, int lane, int status) {
@@ -408,20 +460,21 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
   };
   // Gram-Schmidt of the warp's point; false on a degenerate basis.
   auto gram_schmidt = [&]() -> bool {
-    bool ok;
-    double rmin;
-    const double cancel = mgs_qr(w, V, base, k, g, li, lane, w.phase == kAverage, ok, rmin);
+    const GsResult gs = mgs_qr(V, base, k, lane);
     V = base;  // the orthonormal vectors are in the lower half now
     V1 = base + k * N;
-    if (!ok) return false;
+    if (!gs.ok) return false;
     if (w.phase == kAverage) {
       bool fl = false;
 #pragma unroll
-      for (int i = 0; i < 2; i++) fl = fl || !(w.prod[i] < 1e150 && w.prod[i] > 1e-150);
+      for (int i = 0; i < 2; i++) {
+        w.prod[i] *= gs.r[i];
+        fl = fl || !(w.prod[i] < 1e150 && w.prod[i] > 1e-150);
+      }
       if (__any_sync(FULL, fl)) flush_logs(w);
     }
     if (w.t_gs > 0.0)  // the policy of every adaptive form (renorm.cuh)
-      adaptive::next_renorm_interval(w.L, w.rate_max, (float)cancel, rmin, w.t_gs, tau,
+      adaptive::next_renorm_interval(w.L, w.rate_max, (float)gs.cancel, gs.rmin, w.t_gs, tau,
                                      a.dt_renorm);
     w.t_gs = 0.0;
     return true;
