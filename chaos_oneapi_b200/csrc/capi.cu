@@ -364,19 +364,23 @@ static int ensure_order(chaos_lyap_handle *h, int64_t P) {
   return CHAOS_LYAP_OK;
 }
 
-// A persistent one-lane sweep runs as two launches -- all transients, then the
+// A persistent sweep (one lane or one warp per point) runs as two launches -- all transients, then the
 // averaging phases, those expected to take longest first -- when its points
 // are more than the GPU holds at once (otherwise every point starts at once and
 // the order cannot matter; just above one wave the run is its longest points
 // either way) but few enough waves that the end of the run, where lanes wait
 // for the longest points started last, is a sizeable part of it.  Needs a
-// transient (it is what predicts the cost); the buffers, 48-76 bytes per point,
-// are kept by the handle.  One launch -> two, B200: 256^2 Lorenz points in FP64
+// transient (it is what predicts the cost); the buffers, 48-76 bytes per point
+// (Lorenz-96: 344), are kept by the handle.  One launch -> two, B200: 256^2 Lorenz points in FP64
 // (1.7 waves) 245 -> 195 ms; FP32 Lorenz, 152k points (2 waves) 62 -> 47 ms,
 // 300k 103 -> 85 ms, 1024^2 (14 waves) 309 -> 275 ms; FP32 Rossler, whose
 // longest points take twice the mean, 152k points 82 -> 77 ms; at 1.1 waves of
 // it 55 -> 52 ms.
 constexpr double kTwoPhaseMinWaves = 1.5;
+// The warp-per-point form renormalises each point by itself, so its results do
+// not depend on the order at all: from the first point that has to wait.
+// Lorenz-96, 64^2 points (1.7 waves): 116 -> 94 ms.
+constexpr double kTwoPhaseMinWavesWarp = 1.0;
 constexpr int64_t kTwoPhaseMaxWaves = 32;
 
 // Buffers of a two-launch sweep of P points; *ready false during a stream
@@ -468,9 +472,12 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
       a.queue = h->queue;
       a.queue_stride = chaos::queue_stride_for(P);
       bool two_phase = false;
-      if (!split && m->dim <= 4 && a.t_transient > 0) {
-        const int64_t lanes = chaos::adaptive_resident(m->id, integ, prec, block, variant);
-        if (P >= (int64_t)(kTwoPhaseMinWaves * lanes) && P <= kTwoPhaseMaxWaves * lanes &&
+      const bool warp = m->dim > 4;
+      if (!split && a.t_transient > 0) {
+        const int64_t held = warp ? chaos::l96_resident(integ, prec, d.k)
+                                  : chaos::adaptive_resident(m->id, integ, prec, block, variant);
+        const double least = warp ? kTwoPhaseMinWavesWarp : kTwoPhaseMinWaves;
+        if (held > 0 && P > (int64_t)(least * held) && P <= kTwoPhaseMaxWaves * held &&
             (rc = ensure_resume(h, P, s, &two_phase)))
           return rc;
       }
@@ -479,8 +486,9 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
         a.resume.cost = static_cast<double *>(h->resume);
         a.resume.steps = reinterpret_cast<int64_t *>(a.resume.cost + P);
         a.resume.state = a.resume.steps + P;
-        rc = chaos::launch_adaptive_two_phase(m->id, integ, prec, a, block, variant,
-                                              h->order_scratch, s);
+        rc = warp ? chaos::launch_l96_two_phase(integ, prec, a, h->order_scratch, s)
+                  : chaos::launch_adaptive_two_phase(m->id, integ, prec, a, block, variant,
+                                                     h->order_scratch, s);
         if (rc && rc != chaos::kErrUnsupported) return cuda_fail((cudaError_t)rc, "kernel launch");
         if (!rc) {
           h->last_stream = s;

@@ -125,6 +125,9 @@ int64_t adaptive_resident(int model, int integrator, int precision, int block, i
 inline int64_t resume_state_bytes(int dim, int precision) {
   return (2 * dim + 1) * (precision == kFP32 ? 4 : 8);
 }
+int64_t l96_resident(int integrator, int precision, int k);
+int launch_l96_two_phase(int integrator, int precision, const AdaptiveArgs &a, void *order_scratch,
+                         cudaStream_t s);
 int launch_l96_warp(int integrator, int precision, const AdaptiveArgs &a, int warps_per_block,
                     cudaStream_t s);
 

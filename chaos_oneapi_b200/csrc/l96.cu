@@ -389,15 +389,27 @@ __device__ void finish(Warp &w, const AdaptiveArgs &a, int k, int lane, int stat
   }
 }
 
+// What a launch runs of its points: everything, their transients only (end
+// states into a.resume), or their averaging phases from there.
+enum Mode : int { kWhole = 0, kTransients = 1, kAveraging = 2 };
+
+template <int MODE>
 __device__ __forceinline__ long long fetch(const AdaptiveArgs &a, int lane, long long direct) {
   if (!a.queue) return direct;
-  unsigned long long q = 0;
-  if (lane == 0) q = atomicAdd(a.queue, 1ULL);
-  q = __shfl_sync(FULL, q, 0);
-  if (q >= (unsigned long long)a.P) return a.P;
-  return (long long)((q * (unsigned long long)a.queue_stride) % (unsigned long long)a.P);
+  for (;;) {
+    unsigned long long q = 0;
+    if (lane == 0) q = atomicAdd(a.queue, 1ULL);
+    q = __shfl_sync(FULL, q, 0);
+    if (q >= (unsigned long long)a.P) return a.P;
+    const long long pt =
+        MODE == kAveraging
+            ? (long long)a.order[q]
+            : (long long)((q * (unsigned long long)a.queue_stride) % (unsigned long long)a.P);
+    if (MODE != kAveraging || a.resume.steps[pt] >= 0) return pt;  // else ended in its transient
+  }
 }
 
+template <int MODE>
 __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -417,7 +429,7 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
 
   Warp w;
   long long direct = (long long)blockIdx.x * WARPS + wid;
-  w.pt = fetch(a, lane, direct);
+  w.pt = fetch<MODE>(a, lane, direct);
 
   auto start_tangent = [&]() {
     for (int idx = lane; idx < k * N; idx += 32) V[idx] = (idx / N == idx % N) ? 1.f : 0.f;
@@ -436,26 +448,58 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
   auto start_point = [&]() {
     w.F = (float)a.params.base[w.pt * a.params.ps + 0 * a.params.cs];
     w.gam = (float)a.params.base[w.pt * a.params.ps + 1 * a.params.cs];
+    if constexpr (MODE == kAveraging) {
+      const float *st = static_cast<const float *>(a.resume.state) + w.pt;
 #pragma unroll
-    for (int j = 0; j < C; j++) w.x[j] = (float)a.inits.base[w.pt * a.inits.ps + (li * C + j) * a.inits.cs];
-    w.h = (float)a.h0;
+      for (int j = 0; j < C; j++) {
+        w.x[j] = st[(li * C + j) * a.P];
+        w.kx[j] = st[(N + li * C + j) * a.P];
+      }
+      w.h = st[2 * N * a.P];
+      const long long steps = a.resume.steps[w.pt];
+      w.reject = (steps & kResumeReject) != 0;
+      w.steps = steps & ~kResumeReject;
+    } else {
+#pragma unroll
+      for (int j = 0; j < C; j++)
+        w.x[j] = (float)a.inits.base[w.pt * a.inits.ps + (li * C + j) * a.inits.cs];
+      w.h = (float)a.h0;
+      w.reject = false;
+      w.steps = 0;
+    }
     w.fac_old = 1e-4f;
-    w.reject = false;
-    w.steps = 0;
     w.t_avg = a.t_avg_per_point ? a.t_avg_per_point[w.pt] : a.t_avg;
     w.L = a.dt_renorm / adaptive::kRenormSplitInit;
     w.rate_max = adaptive::initial_renorm_rate(tau, (float)a.dt_renorm);
 #pragma unroll
     for (int i = 0; i < 2; i++) w.sum[i] = w.comp[i] = 0.0, w.prod[i] = 1.0;
-    Jc jc;
-    rhs_state(w.x, w.kx, jc, w.F, w.gam, left, right);
-    if (a.t_transient > 0) {
+    if constexpr (MODE != kAveraging) {
+      Jc jc;
+      rhs_state(w.x, w.kx, jc, w.F, w.gam, left, right);
+    }
+    if (MODE != kAveraging && a.t_transient > 0) {
       w.phase = kTransient;
       w.phase_len = a.t_transient;
       w.t_phase = 0.0;
       w.t_gs = 0.0;
     } else {
       start_tangent();
+    }
+  };
+  // The transient's end state, and the expected cost of the averaging phase.
+  auto save_point = [&]() {
+    float *st = static_cast<float *>(a.resume.state) + w.pt;
+    if (g == 0) {
+#pragma unroll
+      for (int j = 0; j < C; j++) {
+        st[(li * C + j) * a.P] = w.x[j];
+        st[(N + li * C + j) * a.P] = w.kx[j];
+      }
+    }
+    if (lane == 0) {
+      st[2 * N * a.P] = w.h;
+      a.resume.steps[w.pt] = w.steps | (w.reject ? kResumeReject : 0);
+      a.resume.cost[w.pt] = (double)w.steps * (w.t_avg / a.t_transient);
     }
   };
   // Gram-Schmidt of the warp's point; false on a degenerate basis.
@@ -482,7 +526,8 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
 
   if (w.pt < a.P) start_point();
   while (w.pt < a.P) {
-    int status = -1;  // -1: running
+    constexpr int kSaved = 5;
+    int status = -1;  // -1: running; kSaved: the transient is done
     if (w.steps == 0) {  // an initial state outside the escape radius (adaptive.cuh: state_inside)
       bool inside = true;
 #pragma unroll
@@ -495,7 +540,7 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
       const double remaining = w.phase_len - w.t_phase;
       const bool clamped = (double)w.h >= remaining;
       const float h = clamped ? (float)remaining : w.h;
-      const bool joint = w.phase != kTransient;
+      const bool joint = MODE == kAveraging || (MODE == kWhole && w.phase != kTransient);
       w.steps++;
       // state pass: every group computes it; the stage points become J coefficients
       Jc jcs[7];
@@ -573,7 +618,10 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
           if (!__all_sync(FULL, inside)) {
             status = 4;
           } else if (clamped) {
-            if (w.phase == kTransient) {
+            if (MODE == kTransients) {
+              save_point();
+              status = kSaved;
+            } else if (w.phase == kTransient) {
               start_tangent();
             } else if (w.phase == kAlign) {
               if (!gram_schmidt()) status = 1;
@@ -593,8 +641,12 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
       }
     }
     if (status >= 0) {
-      finish(w, a, k, lane, status);
-      w.pt = fetch(a, lane, a.P);
+      if (MODE != kTransients || status != kSaved) finish(w, a, k, lane, status);
+      if (MODE == kTransients && status != kSaved && lane == 0) {
+        a.resume.steps[w.pt] = -1;
+        a.resume.cost[w.pt] = 0.0;
+      }
+      w.pt = fetch<MODE>(a, lane, a.P);
       if (w.pt < a.P) start_point();
     }
   }
@@ -602,27 +654,58 @@ __global__ void __launch_bounds__(WARPS * 32, 4) l96_kernel(const AdaptiveArgs a
 
 }  // namespace l96
 
-int launch_l96_warp(int integrator, int precision, const AdaptiveArgs &a, int, cudaStream_t s) {
+namespace {
+template <int MODE> int64_t l96_blocks(const AdaptiveArgs &a, size_t smem) {
   using namespace l96;
-  if (integrator != kDopri5 || precision != kFP32) return kErrUnsupported;
-  if (a.k < 1 || a.k > N) return kErrUnsupported;
-  const size_t smem = (size_t)WARPS * 2 * a.k * N * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(l96_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  int dev = 0, sms = 0;
+  int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  unsigned grid;
-  if (a.queue) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, l96_kernel, WARPS * 32, smem);
-    grid = (unsigned)std::min<int64_t>((int64_t)std::max(1, per_sm) * sms, (a.P + WARPS - 1) / WARPS);
-  } else {
-    grid = (unsigned)((a.P + WARPS - 1) / WARPS);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, l96_kernel<MODE>, WARPS * 32, smem);
+  return std::min<int64_t>((int64_t)std::max(1, per_sm) * sms, (a.P + WARPS - 1) / WARPS);
+}
+size_t l96_smem(int k) { return (size_t)l96::WARPS * 2 * k * l96::N * sizeof(float); }
+template <int MODE> int launch_l96_mode(const AdaptiveArgs &a, cudaStream_t s) {
+  using namespace l96;
+  const size_t smem = MODE == kTransients ? 0 : l96_smem(a.k);
+  if (smem) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        l96_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
   }
-  l96_kernel<<<grid, WARPS * 32, smem, s>>>(a);
+  const int64_t grid = a.queue ? l96_blocks<MODE>(a, smem) : (a.P + WARPS - 1) / WARPS;
+  l96_kernel<MODE><<<(unsigned)grid, WARPS * 32, smem, s>>>(a);
   return (int)cudaGetLastError();
+}
+bool l96_supported(int integrator, int precision, int k) {
+  return integrator == kDopri5 && precision == kFP32 && k >= 1 && k <= l96::N;
+}
+}  // namespace
+
+int launch_l96_warp(int integrator, int precision, const AdaptiveArgs &a, int, cudaStream_t s) {
+  if (!l96_supported(integrator, precision, a.k)) return kErrUnsupported;
+  return launch_l96_mode<l96::kWhole>(a, s);
+}
+
+int64_t l96_resident(int integrator, int precision, int k) {
+  if (!l96_supported(integrator, precision, k)) return 0;
+  const size_t smem = l96_smem(k);
+  if (cudaFuncSetAttribute(l96::l96_kernel<l96::kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem) != cudaSuccess)
+    return 0;
+  AdaptiveArgs all{};
+  all.P = INT64_MAX / 2;
+  return l96_blocks<l96::kWhole>(all, smem) * l96::WARPS;
+}
+
+int launch_l96_two_phase(int integrator, int precision, const AdaptiveArgs &a, void *order_scratch,
+                         cudaStream_t s) {
+  if (!l96_supported(integrator, precision, a.k)) return kErrUnsupported;
+  int rc = launch_l96_mode<l96::kTransients>(a, s);
+  if (!rc) rc = (int)cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), s);
+  if (!rc)
+    rc = launch_order_longest_first(a.resume.cost, a.P, const_cast<int32_t *>(a.order),
+                                    order_scratch, s);
+  return rc ? rc : launch_l96_mode<l96::kAveraging>(a, s);
 }
 
 }  // namespace chaos
