@@ -66,18 +66,17 @@ __device__ __forceinline__ void mma_slices(uint32_t d, uint64_t a, uint32_t sa, 
              accumulate || j > 0);
 }
 
-// 32 accumulator columns from column c of this warp's lanes.
-__device__ __forceinline__ void load32(uint32_t tmem, int quarter, int c, float (&v)[32]) {
-  uint32_t a[16], b[16];
-  const uint32_t t = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c;
-  tmem_ld16(t, a);
-  tmem_ld16(t + 16, b);
+// kChunk accumulator columns from column c of this warp's lanes.
+constexpr int kChunk = 16;
+__device__ __forceinline__ void load_columns(uint32_t tmem, int quarter, int c,
+                                             float (&v)[kChunk]) {
+  uint32_t a[kChunk / 16][16];
+#pragma unroll
+  for (int i = 0; i < kChunk / 16; i++)
+    tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c + 16 * i), a[i]);
   tmem_wait_ld();
 #pragma unroll
-  for (int j = 0; j < 16; j++) {
-    v[j] = __uint_as_float(a[j]);
-    v[16 + j] = __uint_as_float(b[j]);
-  }
+  for (int j = 0; j < kChunk; j++) v[j] = __uint_as_float(a[j / 16][j % 16]);
 }
 
 struct FwdArgs {
@@ -135,43 +134,73 @@ struct Product {
   }
 };
 
-// Prediction.  Grid (CTAs per network, networks): each CTA strides over tiles
-// of 128 rows with its network's weights resident; a thread takes one row's
-// half of the columns.  Two CTAs per SM, so that one's MMAs run under the
-// other's SiLU epilogue, which bounds the kernel: two special-function
-// operations per unit and row at 16 per cycle and SM, 0.17 ms per 2^18 rows of
-// 4 networks of width 128.  2^20 rows: 1.31 ms (layer by layer: 17.7 ms).
-// Rolled loops: unrolled over the layers, the epilogues waited on instruction
-// fetch.
-template <int W>
-__global__ void __launch_bounds__(kThreads, 2) predict_kernel(const __grid_constant__ FwdArgs g) {
+// Prediction.  Grid (CTAs per network, networks): one CTA per SM with its
+// network's weights resident and kPredictTiles tiles of 128 rows in flight, each
+// with its own 256 threads (a thread takes one row's half of the columns), act
+// buffer, accumulator and barriers, striding over the rows: while one tile waits
+// for its MMAs the others are in their SiLU epilogues, which bound the kernel
+// (two special-function operations per unit and row at 16 per cycle and SM: 0.69
+// ms for 2^20 rows of 4 networks of width 128).  2^20 rows: 1.12 ms (two CTAs
+// per SM with one tile each: 1.31 ms; layer by layer: 17.7 ms).  Rolled loops:
+// unrolled over the layers, the epilogues waited on instruction fetch.
+constexpr int kPredictTiles = 4;
+template <int W> struct PredictSmem {
   using S = Smem<W>;
+  static constexpr int x = S::x, tile = kRows * (kFeat + W) * 2,  // features, activations
+                       bias = x + kPredictTiles * tile, bars = bias + (3 * W + kOutPad) * 4,
+                       bytes = bars + 8 * (1 + kPredictTiles) + 16;
+};
+
+template <int W>
+__global__ void __launch_bounds__(kThreads *kPredictTiles, 1)
+    predict_kernel(const __grid_constant__ FwdArgs g) {
+  using S = Smem<W>;
+  using Q = PredictSmem<W>;
   constexpr int HC = W / 2;  // columns per thread and layer
+  constexpr uint32_t kCols = kPredictTiles * W <= 256 ? 256 : 512;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = smem_u32(smem);
-  float *bias = reinterpret_cast<float *>(smem + S::bias);
-  const uint32_t wbar = base + S::bars, mbar = wbar + 8;
-  uint32_t *slot = reinterpret_cast<uint32_t *>(smem + S::bars + 16);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float *bias = reinterpret_cast<float *>(smem + Q::bias);
+  const int group = threadIdx.x / kThreads, tid = threadIdx.x % kThreads;
+  const uint32_t wbar = base + Q::bars, mbar = wbar + 8 * (1 + group);
+  uint32_t *slot = reinterpret_cast<uint32_t *>(smem + Q::bars + 8 * (1 + kPredictTiles));
+  const int warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, half = warp >> 2;
   const int row = quarter * 32 + lane;  // this thread's row in the epilogues
   const int z = blockIdx.y;
-  if (tid == 0) {
-    mbar_init(wbar, 1);
-    mbar_init(mbar, 1);
+  const uint32_t x = base + Q::x + group * Q::tile, act = x + kRows * kFeat * 2;
+  uint8_t *const xs = smem + Q::x + group * Q::tile, *const as = xs + kRows * kFeat * 2;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i <= kPredictTiles; i++) mbar_init(wbar + 8 * i, 1);
     mbar_init_fence();
     load_weights<W>(g, z, base, wbar);
   }
-  if (warp == 0) tmem_alloc(smem_u32(slot), W);
+  if (threadIdx.x < 32) tmem_alloc(smem_u32(slot), kCols);
   load_biases<W>(g, z, bias);
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  const uint32_t tmem = *slot;
-  Product product{mbar, 0, mbar_wait(wbar, 0)};
+  const uint32_t tmem = *slot + group * W;
+  bool ok = mbar_wait(wbar, 0);
+  uint32_t phase = 0;
+  // Product, for the threads of one tile
+  auto product = [&](uint64_t a, uint64_t b, uint32_t sb, uint32_t idesc, int slices) {
+    fence_proxy_async();
+    fence_before_sync();
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kThreads) : "memory");
+    if (tid == 0) {
+      fence_after_sync();
+      mma_slices(tmem, a, kStepK, b, sb, idesc, slices, false);
+      mma_commit(mbar);
+    }
+    if (ok) ok = mbar_wait(mbar, phase);
+    phase ^= 1;
+    fence_after_sync();
+  };
 
   const int64_t tiles = (g.rows + kRows - 1) / kRows;
-  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  for (int64_t tile = (int64_t)blockIdx.x * kPredictTiles + group; tile < tiles;
+       tile += (int64_t)gridDim.x * kPredictTiles) {
     {  // features: two threads per row, four frequency vectors each
       const int r = tid >> 1, h = tid & 1;
       const int64_t i = tile * kRows + r;
@@ -184,32 +213,32 @@ __global__ void __launch_bounds__(kThreads, 2) predict_kernel(const __grid_const
         q = make_uint4(pack2(sn[0], cs[0]), pack2(sn[1], cs[1]), pack2(sn[2], cs[2]),
                        pack2(sn[3], cs[3]));
       }
-      *reinterpret_cast<uint4 *>(smem + S::x + ((r >> 3) * 2 + h) * 128 + (r & 7) * 16) = q;
+      *reinterpret_cast<uint4 *>(xs + ((r >> 3) * 2 + h) * 128 + (r & 7) * 16) = q;
     }
     // hidden layers: Z = A W; A' = SiLU(Z + b)
 #pragma unroll 1
     for (int l = 0; l < 3; l++) {
-      const uint64_t a = l == 0 ? desc_k(base + S::x, kFeat) : desc_k(base + S::act, W);
+      const uint64_t a = l == 0 ? desc_k(x, kFeat) : desc_k(act, W);
       const uint32_t w = base + (l == 0 ? S::w1 : l == 1 ? S::w2 : S::w3);
-      product(tmem, a, kStepK, desc_mn(w, W), step_mn(W), instr_desc(kRows, W, false, true),
+      product(a, desc_mn(w, W), step_mn(W), instr_desc(kRows, W, false, true),
               l == 0 ? 1 : W / 16);
 #pragma unroll 1
-      for (int c0 = half * HC; c0 < (half + 1) * HC; c0 += 32) {
-        float v[32];
-        load32(tmem, quarter, c0, v);
+      for (int c0 = half * HC; c0 < (half + 1) * HC; c0 += kChunk) {
+        float v[kChunk];
+        load_columns(tmem, quarter, c0, v);
 #pragma unroll
-        for (int c = 0; c < 32; c++) v[c] += bias[l * W + c0 + c];
+        for (int c = 0; c < kChunk; c++) v[c] += bias[l * W + c0 + c];
         silu_chunk(v);
 #pragma unroll
-        for (int c = 0; c < 32; c += 8)
-          *reinterpret_cast<uint4 *>(smem + S::act + ((row >> 3) * (W / 8) + ((c0 + c) >> 3)) * 128 +
+        for (int c = 0; c < kChunk; c += 8)
+          *reinterpret_cast<uint4 *>(as + ((row >> 3) * (W / 8) + ((c0 + c) >> 3)) * 128 +
                                      (row & 7) * 16) =
               make_uint4(pack2(v[c], v[c + 1]), pack2(v[c + 2], v[c + 3]),
                          pack2(v[c + 4], v[c + 5]), pack2(v[c + 6], v[c + 7]));
       }
     }
-    product(tmem, desc_k(base + S::act, W), kStepK, desc_mn(base + S::w4, kOutPad),
-            step_mn(kOutPad), instr_desc(kRows, kOutPad, false, true), W / 16);
+    product(desc_k(act, W), desc_mn(base + S::w4, kOutPad), step_mn(kOutPad),
+            instr_desc(kRows, kOutPad, false, true), W / 16);
     const int64_t i = tile * kRows + row;
     if (half == 0) {
       uint32_t a[16];
@@ -228,10 +257,10 @@ __global__ void __launch_bounds__(kThreads, 2) predict_kernel(const __grid_const
       }
     }
   }
-  if (!product.ok && lane == 0) atomicExch(g.P.err, 1);
+  if (!ok && lane == 0) atomicExch(g.P.err, 1);
   fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, W);
+  if (threadIdx.x < 32) tmem_dealloc(*slot, kCols);
 }
 
 // Training: the forward pass of kTrainRows = 64 rows of one network, the loss
@@ -695,8 +724,8 @@ template <class K> int allow_smem(K kern, int bytes, std::atomic<uint64_t> &seen
 
 template <int W> int launch_predict(const FwdArgs &a, unsigned gx, cudaStream_t s) {
   static std::atomic<uint64_t> seen{0};
-  if (int rc = allow_smem(predict_kernel<W>, Smem<W>::bytes, seen)) return rc;
-  predict_kernel<W><<<dim3(gx, a.P.E), kThreads, Smem<W>::bytes, s>>>(a);
+  if (int rc = allow_smem(predict_kernel<W>, PredictSmem<W>::bytes, seen)) return rc;
+  predict_kernel<W><<<dim3(gx, a.P.E), kThreads * kPredictTiles, PredictSmem<W>::bytes, s>>>(a);
   return (int)cudaGetLastError();
 }
 
@@ -747,8 +776,9 @@ int fused_predict(const Params &P, const FeatureMap &f, const double *xy, int64_
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t per_net = std::max(1, 2 * sms / P.E);
-  const unsigned gx = (unsigned)std::min<int64_t>(per_net, (rows + kRows - 1) / kRows);
+  const int64_t per_net = std::max(1, sms / P.E);
+  const int64_t need = (rows + kRows * kPredictTiles - 1) / (kRows * kPredictTiles);
+  const unsigned gx = (unsigned)std::min<int64_t>(per_net, need);
   return P.W == 128 ? launch_predict<128>(a, gx, s) : launch_predict<64>(a, gx, s);
 }
 

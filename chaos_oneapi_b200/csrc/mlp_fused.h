@@ -121,13 +121,20 @@ __device__ __forceinline__ float divide_above_one(float z, float d) {
   const float q = z * r;
   return fmaf(fmaf(-q, d, z), r, q);
 }
+// 1 + e^-z as 1 + 2^(-z log2 e).  Denormal powers may flush to zero: the sum is
+// 1 either way, and the instruction needs no scaling around it.
+__device__ __forceinline__ float one_plus_exp_neg(float z) {
+  float e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-z * 1.44269504088896341f));
+  return 1.f + e;
+}
 // v[i] = SiLU(v[i]), and v[i] = u[i] SiLU'(v[i]): the values of silu / dsilu.
 template <int N> __device__ __forceinline__ void silu_chunk(float (&v)[N]) {
   float q[N];
   bool fast = true;
 #pragma unroll
   for (int i = 0; i < N; i++) {
-    const float d = 1.f + __expf(-v[i]);
+    const float d = one_plus_exp_neg(v[i]);
     fast = fast && d < kFastDivLimit;  // false for NaN
     q[i] = divide_above_one(v[i], d);
   }
@@ -152,7 +159,7 @@ __device__ __forceinline__ void dsilu_chunk(const float (&u)[N], float (&v)[N]) 
   bool fast = true;
 #pragma unroll
   for (int i = 0; i < N; i++) {
-    const float d = 1.f + __expf(-v[i]);
+    const float d = one_plus_exp_neg(v[i]);
     fast = fast && d < kFastDivLimit;
     const float sg = divide_above_one(1.f, d);
     q[i] = u[i] * (sg * (1.f + v[i] * (1.f - sg)));
