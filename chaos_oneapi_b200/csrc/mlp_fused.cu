@@ -109,7 +109,7 @@ __device__ __forceinline__ void load_weights(const FwdArgs &g, int z, uint32_t b
 template <int W>
 __device__ __forceinline__ void load_biases(const FwdArgs &g, int z, float *bias) {
   const float *p = g.P.p + z * g.P.np;
-  for (int i = threadIdx.x; i < 3 * W + kOutPad; i += kThreads)
+  for (int i = threadIdx.x; i < 3 * W + kOutPad; i += blockDim.x)
     bias[i] = __ldcg(p + (i < 3 * W ? g.P.off_b[i / W] + i % W : g.P.off_b[3] + i - 3 * W));
 }
 
@@ -272,20 +272,20 @@ __global__ void __launch_bounds__(kThreads *kPredictTiles, 1)
 // epilogue and a 1024-row batch of 4 networks spreads over 64 SMs.  The
 // pre-activations of the hidden layers stay in tensor memory (columns 0 .. 3 W)
 // for the backward pass.  A step of 1024 rows and 4 networks of width 128, this
-// kernel and gradient_kernel: 30 us (24 launches, layer by layer: 530 us).
-constexpr int kTrainRows = 64;
+// kernel and gradient_kernel: 22 us (24 launches, layer by layer: 530 us).
+constexpr int kTrainRows = 64, kTrainThreads = 512;
 
 template <int W>
-__global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constant__ FwdArgs g) {
+__global__ void __launch_bounds__(kTrainThreads, 1) train_kernel(const __grid_constant__ FwdArgs g) {
   using S = Smem<W>;
-  constexpr int HC = W / 2;
+  constexpr int HC = W / 4;  // columns per thread and layer
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = smem_u32(smem);
   float *bias = reinterpret_cast<float *>(smem + S::bias);
   const uint32_t wbar = base + S::bars, mbar = wbar + 8;
   uint32_t *slot = reinterpret_cast<uint32_t *>(smem + S::bars + 16);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, half = warp >> 2;
+  const int quarter = warp & 3, part = warp >> 2;
   const int z = blockIdx.y;
   const int64_t tile = blockIdx.x;
   const int64_t padded = (g.rows + kRows - 1) / kRows * kRows;  // rows of a buffer per network
@@ -300,21 +300,20 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
     mbar_init_fence();
   }
   if (warp == 0) tmem_alloc(smem_u32(slot), 4 * W);
-  // features: four threads per row, two frequency vectors each
-  const int fr = tid >> 2, fh = tid & 3;
+  // features: eight threads per row, one frequency vector each
+  const int fr = tid >> 3, fh = tid & 7;
   const int64_t fi = tile * kTrainRows + fr;
-  uint2 fq = make_uint2(0, 0);
+  uint32_t fq = 0;
   if (fi < g.rows) {
-    float u, v, sn[2], cs[2];
+    float u, v, sn, cs;
     normalised(g.f, g.xy, g.idx ? (int64_t)g.idx[fi] : fi, u, v);
-#pragma unroll
-    for (int f = 0; f < 2; f++) feature_pair(g.f, u, v, 2 * fh + f, sn[f], cs[f]);
-    fq = make_uint2(pack2(sn[0], cs[0]), pack2(sn[1], cs[1]));
+    feature_pair(g.f, u, v, fh, sn, cs);
+    fq = pack2(sn, cs);
   }
+  const int fin = (fr & 7) * 16 + (fh & 3) * 4;
   {  // row r of the tile is row (r / 16) * 32 + r % 16 of the MMA
     const int mg = (fr >> 4) * 4 + ((fr >> 3) & 1);
-    *reinterpret_cast<uint2 *>(smem + S::x + (mg * 2 + (fh >> 1)) * 128 + (fr & 7) * 16 +
-                               (fh & 1) * 8) = fq;
+    *reinterpret_cast<uint32_t *>(smem + S::x + (mg * 2 + (fh >> 2)) * 128 + fin) = fq;
   }
   // this thread's rows in the epilogues, r0 and r0 + 8, and their targets
   const int r0 = quarter * 16 + (lane >> 2), cp = (lane & 3) * 2;
@@ -323,12 +322,12 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const int c = (j >> 1) * 8 + cp + (j & 1);
-    ti[j] = half == 0 && c < outs ? g.tinv[c] : 0.f;
+    ti[j] = part == 0 && c < outs ? g.tinv[c] : 0.f;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int64_t i = tile * kTrainRows + r0 + 8 * q;
       tc[q][j] = 0.f;
-      if (half == 0 && c < outs && i < g.rows) {
+      if (part == 0 && c < outs && i < g.rows) {
         const int64_t k = g.idx ? (int64_t)g.idx[i] : i;
         tc[q][j] = (float)g.T[k * outs + c] - g.tmean[c];
       }
@@ -339,9 +338,8 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
   if (tid == 0) load_weights<W>(g, z, base, wbar);
   load_biases<W>(g, z, bias);
   if (z == 0)
-    *reinterpret_cast<uint2 *>(reinterpret_cast<uint8_t *>(g.b.X) +
-                               ((fi >> 3) * 2 + (fh >> 1)) * 128 + (fr & 7) * 16 +
-                               (fh & 1) * 8) = fq;
+    *reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(g.b.X) +
+                                  ((fi >> 3) * 2 + (fh >> 2)) * 128 + fin) = fq;
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -350,10 +348,11 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
   Product product{mbar, 0, mbar_wait(wbar, 0)};
   const int64_t row0 = z * padded + tile * kTrainRows;  // the tile's first row in the buffers
 
-  // 32 columns from c0: the next operand, and the same core matrices outside
-  auto store32 = [&](int c0, const float (&v)[16], bf16 *out) {
+  // this thread's columns from c0: the next operand, and the same core matrices
+  // outside
+  auto store = [&](int c0, const float (&v)[HC / 2], bf16 *out) {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < HC / 8; i++)
 #pragma unroll
       for (int q = 0; q < 2; q++) {
         const uint32_t x = pack2(v[4 * i + 2 * q], v[4 * i + 2 * q + 1]);
@@ -365,16 +364,17 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
                                       in) = x;
       }
   };
-  auto load = [&](uint32_t col, float (&v)[16]) {
-    uint32_t a[16];
-    tmem_ld_16x32(tmem + lanes + col, a);
+  auto load = [&](uint32_t col, float (&v)[HC / 2]) {
+    uint32_t a[HC / 2];
+    if constexpr (HC == 32) tmem_ld_16x32(tmem + lanes + col, a);
+    else tmem_ld_16x16(tmem + lanes + col, a);
     tmem_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = __uint_as_float(a[j]);
+    for (int j = 0; j < HC / 2; j++) v[j] = __uint_as_float(a[j]);
   };
-  auto add_bias = [&](int c, float (&v)[16]) {
+  auto add_bias = [&](int c, float (&v)[HC / 2]) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < HC / 8; i++) {
       const float2 b = *reinterpret_cast<const float2 *>(bias + c + 8 * i + cp);
       v[4 * i] += b.x;
       v[4 * i + 1] += b.y;
@@ -382,6 +382,7 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
       v[4 * i + 3] += b.y;
     }
   };
+  const int c0 = part * HC;
 
   // hidden layers: Z = A W; A' = SiLU(Z + b)
 #pragma unroll 1
@@ -391,21 +392,18 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
     product(tmem + l * W, a, kStepK, desc_mn(w, W), step_mn(W), instr_desc(kRows, W, false, true),
             l == 0 ? 1 : W / 16);
     bf16 *out = l == 0 ? g.b.A[0] : l == 1 ? g.b.A[1] : g.b.A[2];
-#pragma unroll 1
-    for (int c0 = half * HC; c0 < (half + 1) * HC; c0 += 32) {
-      float v[16];
-      load(l * W + c0, v);
-      add_bias(l * W + c0, v);
-      silu_chunk(v);
-      store32(c0, v, out);
-    }
+    float v[HC / 2];
+    load(l * W + c0, v);
+    add_bias(l * W + c0, v);
+    silu_chunk(v);
+    store(c0, v, out);
   }
   // output layer, loss and its gradient dY = 2 (Y - T) / (rows outs), zero on
   // the padding and past the rows
   const uint32_t dy = tmem + 3 * W;
   product(dy, desc_k(base + S::act, W), kStepK, desc_mn(base + S::w4, kOutPad), step_mn(kOutPad),
           instr_desc(kRows, kOutPad, false, true), W / 16);
-  if (half == 0) {
+  if (part == 0) {
     uint32_t a[8];
     tmem_ld_16x16(dy + lanes, a);
     tmem_wait_ld();
@@ -450,15 +448,12 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(const __grid_constan
                               : desc_k(base + (l == 1 ? S::w3 : S::w2), W);
     product(dy, a, kStepK, w, kStepK, instr_desc(kRows, W), l == 2 ? 1 : W / 16);
     bf16 *out = l == 0 ? g.b.dZ[0] : l == 1 ? g.b.dZ[1] : g.b.dZ[2];
-#pragma unroll 1
-    for (int c0 = half * HC; c0 < (half + 1) * HC; c0 += 32) {
-      float da[16], v[16];
-      load(3 * W + c0, da);
-      load(l * W + c0, v);
-      add_bias(l * W + c0, v);
-      dsilu_chunk(da, v);
-      store32(c0, v, out);
-    }
+    float da[HC / 2], v[HC / 2];
+    load(3 * W + c0, da);
+    load(l * W + c0, v);
+    add_bias(l * W + c0, v);
+    dsilu_chunk(da, v);
+    store(c0, v, out);
   }
   if (!product.ok && lane == 0) atomicExch(g.P.err, 1);
   fence_before_sync();
@@ -497,11 +492,14 @@ template <int W> struct GradSmem {
 // dW = A^T dZ over all rows, 128 at a time, in row order, accumulated in tensor
 // memory (both operands MN-major: K runs over the rows); the first layer's
 // gradient transposed (dZ^T X), so that M is the network's width.  Tiles arrive
-// by bulk copies, kStages of them in flight: the kernel's time is a CTA's reads
-// of A from L2 and the chain of its epilogue, which is why the square matrices
-// are cut into slices (a whole one took 24 us for Adam's 64 elements per
-// thread).  The epilogue applies Adam to the elements it holds, read ahead
-// before the products are waited for.
+// by bulk copies, kStages of them in flight, one copy per lane of a warp; the
+// kernel's time is a CTA's reads of A from L2 (40 KB per tile) and the chain of
+// its epilogue, which is why the square matrices are cut into slices.  The
+// epilogue applies Adam through shared memory, consecutive threads on consecutive
+// parameters (a lane per row of the accumulator, 32 lines per access, took four
+// times as long), the first parameters and moments read ahead: the step before
+// the previous kernel wrote them, and they come from L2, past any older line of
+// this SM's first-level cache.
 template <int W>
 __device__ void weight_gradient(const GradArgs &g, int l, int n0, int z, uint8_t *smem) {
   using S = GradSmem<W>;
@@ -523,20 +521,24 @@ __device__ void weight_gradient(const GradArgs &g, int l, int n0, int z, uint8_t
     mbar_init_fence();
   }
   if (warp == 0) tmem_alloc(smem_u32(slot), 32);
-  // this thread's elements of the epilogue, row m, 16 columns from c0
-  const int m = quarter * 32 + lane, c0 = half * 16;
-  const bool mine = quarter * 32 < W && c0 < N;
+  // The epilogue's elements, four consecutive ones of a gradient row at a time:
+  // quad q is row r, columns c .. c + 3 of a matrix of `cols` columns.  Quads of
+  // consecutive threads are consecutive in memory.  The first quad's parameter
+  // and moments are read ahead.
   const int64_t w0 = z * g.P.np + g.P.off_w[l];
-  const int cols = square ? W : 16;
-  float p[16], mo[16], ve[16];
-  if (mine && g.adam) {
-#pragma unroll
-    for (int c = 0; c < 16; c++) {
-      const int64_t i = l == 0 ? w0 + (int64_t)c * W + m : w0 + (int64_t)m * cols + n0 + c0 + c;
-      p[c] = __ldcg(g.P.p + i);
-      mo[c] = __ldcg(g.P.m + i);
-      ve[c] = __ldcg(g.P.v + i);
-    }
+  const int cols = square || l == 0 ? W : kOutPad;
+  const int per_row = (l == 0 ? W : N) / 4, quads = W * N / 4;
+  auto row_of = [&](int q) { return q / per_row; };
+  auto col_of = [&](int q) { return (square ? n0 : 0) + q % per_row * 4; };
+  auto at = [&](int q) { return w0 + (int64_t)row_of(q) * cols + col_of(q); };
+  auto read = [&](const float *src, int q) {
+    return __ldcg(reinterpret_cast<const float4 *>(src + at(q)));
+  };
+  float4 p, mo, ve;
+  if (g.adam && tid < quads) {
+    p = read(g.P.p, tid);
+    mo = read(g.P.m, tid);
+    ve = read(g.P.v, tid);
   }
   wait_previous();
   launch_dependents();
@@ -545,22 +547,25 @@ __device__ void weight_gradient(const GradArgs &g, int l, int n0, int z, uint8_t
   fence_after_sync();
   const uint32_t tmem = *slot;
   int *flag = reinterpret_cast<int *>(slot + 1);
-  if (tid == 0) {
+  if (warp == 1) {  // loads, one copy per lane
     bool ok = true;
-    auto load = [&](int64_t t) {
+    for (int64_t t = 0; t < tiles; t++) {
       const int st = (int)(t % kStages);
       const uint32_t bar = full + 8 * st, sa = base + st * S::stage;
-      mbar_expect_tx(bar, bytes_a + bytes_b);
-      bulk_load(sa, a + t * kRows * W, bytes_a, bar);
-      if (square) {  // the slice's core matrices, row group by row group
-        for (int rg = 0; rg < kRows / 8; rg++)
-          bulk_load(sa + S::mat + rg * kSlice * 16,
-                    b + (t * (kRows / 8) + rg) * W * 8 + n0 * 8, kSlice * 16, bar);
-      } else {
-        bulk_load(sa + S::mat, b + t * kRows * N, bytes_b, bar);
-      }
-    };
-    for (int64_t t = 0; t < tiles && t < kStages; t++) load(t);
+      // the MMAs of the stage's last tile
+      if (t >= kStages && ok) ok = mbar_wait(done + 8 * st, (uint32_t)((t / kStages - 1) & 1));
+      if (lane == 0) mbar_expect_tx(bar, bytes_a + bytes_b);
+      __syncwarp();
+      if (lane == 16) bulk_load(sa, a + t * kRows * W, bytes_a, bar);
+      if (square && lane < kRows / 8)  // the slice's core matrices, row group by row group
+        bulk_load(sa + S::mat + lane * kSlice * 16,
+                  b + (t * (kRows / 8) + lane) * W * 8 + n0 * 8, kSlice * 16, bar);
+      if (!square && lane == 0) bulk_load(sa + S::mat, b + t * kRows * N, bytes_b, bar);
+    }
+    if (!ok && lane == 0) atomicExch(g.P.err, 1);
+  }
+  if (tid == 0) {
+    bool ok = true;
     const uint32_t idesc = instr_desc(kRows, N, true, true);
     for (int64_t t = 0; t < tiles; t++) {
       const int st = (int)(t % kStages);
@@ -569,12 +574,6 @@ __device__ void weight_gradient(const GradArgs &g, int l, int n0, int z, uint8_t
       mma_slices(tmem, desc_mn(sa, W), step_mn(W), desc_mn(sa + S::mat, N), step_mn(N), idesc,
                  kRows / 16, t > 0);
       mma_commit(done + 8 * st);
-      // refill the stage of the tile before this one, once its MMAs are done
-      if (t > 0 && t - 1 + kStages < tiles) {
-        const int64_t u = t - 1;
-        if (ok) ok = mbar_wait(done + 8 * (int)(u % kStages), (uint32_t)((u / kStages) & 1));
-        load(u + kStages);
-      }
     }
     // thread 0 waits for the last tile's MMAs (its commit covers all before
     // it); the barrier after that releases the others, who have not followed
@@ -587,43 +586,51 @@ __device__ void weight_gradient(const GradArgs &g, int l, int n0, int z, uint8_t
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  if (mine && *flag) {  // rows beyond W are the next rows' bytes read as features
+  // accumulator -> shared memory (over the first stage), lane = row m; rows
+  // beyond W are the next rows' bytes read as features
+  constexpr int pitch = kSlice + 4;
+  float *const acc = reinterpret_cast<float *>(smem);
+  const bool ready = *flag != 0;
+  if (quarter * 32 < W && half * 16 < N) {
     uint32_t v[16];
-    tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
+    tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 16), v);
     tmem_wait_ld();
-    if (!g.adam) {
+    float4 *d = reinterpret_cast<float4 *>(acc + (quarter * 32 + lane) * pitch + half * 16);
 #pragma unroll
-      for (int c = 0; c < 16; c++)
-        g.P.g[l == 0 ? w0 + (int64_t)c * W + m : w0 + (int64_t)m * cols + n0 + c0 + c] =
-            __uint_as_float(v[c]);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 16; c++)
-        p[c] = adam_update(p[c], __uint_as_float(v[c]), mo[c], ve[c], g.a.lr, g.a.b1, g.a.b2,
-                           g.a.eps, g.a.c1, g.a.c2);
-      if (l == 0) {
-#pragma unroll
-        for (int c = 0; c < 16; c++) {
-          const int64_t i = w0 + (int64_t)c * W + m;
-          g.P.p[i] = p[c];
-          g.P.m[i] = mo[c];
-          g.P.v[i] = ve[c];
-          g.P.pb[w0 + core_index(c, m, W)] = __float2bfloat16(p[c]);
-        }
-      } else {
-        const int64_t i = w0 + (int64_t)m * cols + n0 + c0;
-#pragma unroll
-        for (int c = 0; c < 16; c += 4) {
-          *reinterpret_cast<float4 *>(g.P.p + i + c) = make_float4(p[c], p[c + 1], p[c + 2], p[c + 3]);
-          *reinterpret_cast<float4 *>(g.P.m + i + c) = make_float4(mo[c], mo[c + 1], mo[c + 2], mo[c + 3]);
-          *reinterpret_cast<float4 *>(g.P.v + i + c) = make_float4(ve[c], ve[c + 1], ve[c + 2], ve[c + 3]);
-        }
-#pragma unroll
-        for (int c = 0; c < 16; c += 8)
-          *reinterpret_cast<uint4 *>(g.P.pb + w0 + core_index(m, n0 + c0 + c, cols)) =
-              make_uint4(pack2(p[c], p[c + 1]), pack2(p[c + 2], p[c + 3]),
-                         pack2(p[c + 4], p[c + 5]), pack2(p[c + 6], p[c + 7]));
+    for (int c = 0; c < 4; c++)
+      d[c] = make_float4(__uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]),
+                         __uint_as_float(v[4 * c + 2]), __uint_as_float(v[4 * c + 3]));
+  }
+  __syncthreads();
+  // Rolled: it runs once per launch, so its instructions are fetched cold.
+  if (ready) {
+#pragma unroll 1
+    for (int q = tid; q < quads; q += kThreads) {
+      float4 pn = p, mn = mo, vn = ve;
+      if (g.adam && q + kThreads < quads) {
+        pn = read(g.P.p, q + kThreads);
+        mn = read(g.P.m, q + kThreads);
+        vn = read(g.P.v, q + kThreads);
       }
+      const int r = row_of(q), c = q % per_row * 4;
+      const float4 d = l == 0 ? make_float4(acc[c * pitch + r], acc[(c + 1) * pitch + r],
+                                            acc[(c + 2) * pitch + r], acc[(c + 3) * pitch + r])
+                              : *reinterpret_cast<const float4 *>(acc + r * pitch + c);
+      if (!g.adam) {
+        *reinterpret_cast<float4 *>(g.P.g + at(q)) = d;
+        continue;
+      }
+      const AdamStep &s = g.a;
+      p.x = adam_update(p.x, d.x, mo.x, ve.x, s.lr, s.b1, s.b2, s.eps, s.c1, s.c2);
+      p.y = adam_update(p.y, d.y, mo.y, ve.y, s.lr, s.b1, s.b2, s.eps, s.c1, s.c2);
+      p.z = adam_update(p.z, d.z, mo.z, ve.z, s.lr, s.b1, s.b2, s.eps, s.c1, s.c2);
+      p.w = adam_update(p.w, d.w, mo.w, ve.w, s.lr, s.b1, s.b2, s.eps, s.c1, s.c2);
+      *reinterpret_cast<float4 *>(g.P.p + at(q)) = p;
+      *reinterpret_cast<float4 *>(g.P.m + at(q)) = mo;
+      *reinterpret_cast<float4 *>(g.P.v + at(q)) = ve;
+      *reinterpret_cast<uint2 *>(g.P.pb + w0 + core_index(r, col_of(q), cols)) =
+          make_uint2(pack2(p.x, p.y), pack2(p.z, p.w));
+      p = pn, mo = mn, ve = vn;
     }
   }
   fence_before_sync();
@@ -631,83 +638,104 @@ __device__ void weight_gradient(const GradArgs &g, int l, int n0, int z, uint8_t
   if (warp == 0) tmem_dealloc(tmem, 32);
 }
 
-// Bias vector l of network z: db[c] = the sum of dZ's column c over the rows,
-// in row order (one chain of additions per column, the rows read 16 ahead).
-// Tiles are turned row-major in shared memory (pitch padded by 16 bytes: no
-// bank conflicts either way), two buffers, the next tile's loads in flight.
-template <int C>
-__device__ void bias_gradient(const GradArgs &g, const bf16 *src, int64_t i0, uint8_t *smem) {
-  constexpr int kChunks = kRows * C / 8, U = kChunks / kThreads;
-  static_assert(kChunks % kThreads == 0, "whole chunks per thread");
-  constexpr int pitch = C * 2 + 16;
-  const int tid = threadIdx.x;
+// Columns n0 .. n0 + 31 (of the output layer: all 16) of bias vector l of
+// network z: db[c] = the sum of dZ's column c over the rows, in row order -- one
+// chain of additions per column, a lane each, straight from the tiles' core
+// matrices in shared memory (the copies of kBiasTiles tiles in flight).
+constexpr int kBiasTiles = 8;
+template <int C, int NC>
+__device__ void bias_gradient(const GradArgs &g, const bf16 *src, int n0, int64_t i0,
+                              uint8_t *smem) {
+  constexpr int kTile = kRows * NC * 2, kBars = kBiasTiles * kTile;
+  const uint32_t base = smem_u32(smem), full = base + kBars;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t tiles = (g.rows + kRows - 1) / kRows;
+  if (tid == 0) {
+    for (int i = 0; i < kBiasTiles; i++) mbar_init(full + 8 * i, 1);
+    mbar_init_fence();
+  }
   wait_previous();
   launch_dependents();
-  uint4 q[U];
-  auto fetch = [&](int64_t t) {
-    const uint4 *s = reinterpret_cast<const uint4 *>(src + t * kRows * C);
-#pragma unroll
-    for (int u = 0; u < U; u++) q[u] = __ldcg(s + u * kThreads + tid);
-  };
-  fetch(0);
+  __syncthreads();
   float s = 0.f;
-  for (int64_t t = 0; t < tiles; t++) {
-    uint8_t *buf = smem + (t & 1) * kRows * pitch;
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int k = u * kThreads + tid, core = k >> 3;
-      const int r = (core / (C / 8)) * 8 + (k & 7), cg = core % (C / 8);
-      *reinterpret_cast<uint4 *>(buf + r * pitch + cg * 16) = q[u];
-    }
-    __syncthreads();  // the other buffer's readers are done as well
-    if (t + 1 < tiles) fetch(t + 1);
-    if (tid < C) {
-      const int n = (int)min((int64_t)kRows, g.rows - t * kRows);
-      const uint8_t *col = buf + tid * 2;
-      auto at = [&](int r) { return __bfloat162float(*reinterpret_cast<const bf16 *>(col + r * pitch)); };
-      int r = 0;
-      if (n >= 16) {
-        float x[16], y[16];
-#pragma unroll
-        for (int j = 0; j < 16; j++) x[j] = at(j);
-        for (r = 16; r + 16 <= n; r += 16) {
-#pragma unroll
-          for (int j = 0; j < 16; j++) y[j] = at(r + j);
-#pragma unroll
-          for (int j = 0; j < 16; j++) s += x[j];
-#pragma unroll
-          for (int j = 0; j < 16; j++) x[j] = y[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 16; j++) s += x[j];
+  bool ok = true;
+  for (int64_t t0 = 0; t0 < tiles; t0 += kBiasTiles) {
+    const uint32_t parity = (uint32_t)((t0 / kBiasTiles) & 1);
+    const int nt = (int)min((int64_t)kBiasTiles, tiles - t0);
+    if (warp == 1) {
+      for (int t = 0; t < nt; t++) {
+        const uint32_t bar = full + 8 * t, dst = base + t * kTile;
+        if (lane == 0) mbar_expect_tx(bar, kTile);
+        __syncwarp();
+        if (lane < kRows / 8)  // the columns' core matrices, row group by row group
+          bulk_load(dst + lane * NC * 16, src + ((t0 + t) * (kRows / 8) + lane) * C * 8 + n0 * 8,
+                    NC * 16, bar);
       }
-      for (; r < n; r++) s += at(r);
+    } else if (warp == 0) {
+      for (int t = 0; t < nt; t++) {
+        if (ok) ok = mbar_wait(full + 8 * t, parity);
+        const int n = (int)min((int64_t)kRows, g.rows - (t0 + t) * kRows);
+        const uint8_t *col = smem + t * kTile + (lane >> 3) * 128 + (lane & 7) * 2;
+        auto at = [&](int j) {  // row j of 16 at col
+          return __bfloat162float(
+              *reinterpret_cast<const bf16 *>(col + (j >> 3) * NC * 16 + (j & 7) * 16));
+        };
+        if (lane < NC) {
+          int left = n;
+          if (left >= 16) {  // 16 rows read ahead of the 16 being added
+            float x[16], y[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) x[j] = at(j);
+            col += 2 * NC * 16;
+#pragma unroll 1
+            for (left -= 16; left >= 16; left -= 16, col += 2 * NC * 16) {
+#pragma unroll
+              for (int j = 0; j < 16; j++) y[j] = at(j);
+#pragma unroll
+              for (int j = 0; j < 16; j++) s += x[j];
+#pragma unroll
+              for (int j = 0; j < 16; j++) x[j] = y[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; j++) s += x[j];
+          }
+          for (int j = 0; j < left; j++) s += at(j);
+        }
+      }
     }
+    if (t0 + kBiasTiles < tiles) __syncthreads();  // the buffers are free again
   }
-  if (tid < C) {
-    apply(g, i0 + tid, s);
-    if (g.adam) g.P.pb[i0 + tid] = __float2bfloat16(g.P.p[i0 + tid]);
+  if (warp == 0) {
+    if (!ok && lane == 0) atomicExch(g.P.err, 1);
+    if (ok && lane < NC) {
+      apply(g, i0 + n0 + lane, s);
+      if (g.adam) g.P.pb[i0 + n0 + lane] = __float2bfloat16(g.P.p[i0 + n0 + lane]);
+    }
   }
 }
 
-// blockIdx.y: network; blockIdx.x: the first and last weight matrix, the
-// slices of the two square ones, then the bias vectors.
+// blockIdx.y: network; blockIdx.x: the slices of the two square weight matrices,
+// the first and last one, then the bias vectors in pieces of 32 columns.
+template <int W> struct GradGrid {
+  static constexpr int slices = W / kSlice, weights = 2 + 2 * slices, pieces = W / 32,
+                       blocks = weights + 3 * pieces + 1;
+};
 template <int W>
 __global__ void __launch_bounds__(kThreads, 1) gradient_kernel(const __grid_constant__ GradArgs g) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int kSlices = W / kSlice, kWeights = 2 + 2 * kSlices;
+  using B = GradGrid<W>;
   const int z = blockIdx.y, x = blockIdx.x;
   const int64_t tiles = (g.rows + kRows - 1) / kRows;
-  if (x < 2 * kSlices) {
-    weight_gradient<W>(g, 1 + x / kSlices, x % kSlices * kSlice, z, smem);
-  } else if (x < kWeights) {
-    weight_gradient<W>(g, x == 2 * kSlices ? 0 : 3, 0, z, smem);
+  if (x < 2 * B::slices) {
+    weight_gradient<W>(g, 1 + x / B::slices, x % B::slices * kSlice, z, smem);
+  } else if (x < B::weights) {
+    weight_gradient<W>(g, x == 2 * B::slices ? 0 : 3, 0, z, smem);
+  } else if (x < B::blocks - 1) {
+    const int l = (x - B::weights) / B::pieces, n0 = (x - B::weights) % B::pieces * 32;
+    bias_gradient<W, 32>(g, g.b.dZ[l] + z * tiles * kRows * W, n0, z * g.P.np + g.P.off_b[l], smem);
   } else {
-    const int l = x - kWeights;
-    const int64_t i0 = z * g.P.np + g.P.off_b[l];
-    if (l < 3) bias_gradient<W>(g, g.b.dZ[l] + z * tiles * kRows * W, i0, smem);
-    else bias_gradient<kOutPad>(g, g.b.dY + z * tiles * kRows * kOutPad, i0, smem);
+    bias_gradient<kOutPad, kOutPad>(g, g.b.dY + z * tiles * kRows * kOutPad, 0,
+                                    z * g.P.np + g.P.off_b[3], smem);
   }
 }
 
@@ -734,13 +762,14 @@ template <int W> int launch_predict(const FwdArgs &a, unsigned gx, cudaStream_t 
 // with the programmatic-dependency attribute, the preamble and the launch
 // itself overlap the previous kernel's end.
 template <class Args>
-int launch_dependent(void (*kern)(Args), dim3 grid, int smem, cudaStream_t s, const Args &args) {
+int launch_dependent(void (*kern)(Args), dim3 grid, int threads, int smem, cudaStream_t s,
+                     const Args &args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
@@ -752,13 +781,13 @@ template <int W> int launch_train(const FwdArgs &a, cudaStream_t s) {
   if (int rc = allow_smem(train_kernel<W>, Smem<W>::bytes, seen)) return rc;
   // whole 128-row tiles: gradient_kernel reads the padding rows (zeros)
   const dim3 grid((unsigned)(train_tiles(a.rows) * (kRows / kTrainRows)), a.P.E);
-  return launch_dependent<FwdArgs>(train_kernel<W>, grid, Smem<W>::bytes, s, a);
+  return launch_dependent<FwdArgs>(train_kernel<W>, grid, kTrainThreads, Smem<W>::bytes, s, a);
 }
 template <int W> int launch_gradient(const GradArgs &a, cudaStream_t s) {
   static std::atomic<uint64_t> seen{0};
   if (int rc = allow_smem(gradient_kernel<W>, GradSmem<W>::bytes, seen)) return rc;
-  return launch_dependent<GradArgs>(gradient_kernel<W>, dim3(2 + 2 * (W / kSlice) + 4, a.P.E),
-                                    GradSmem<W>::bytes, s, a);
+  return launch_dependent<GradArgs>(gradient_kernel<W>, dim3(GradGrid<W>::blocks, a.P.E),
+                                    kThreads, GradSmem<W>::bytes, s, a);
 }
 
 }  // namespace
