@@ -231,8 +231,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 1)
 
 }  // namespace adaptive
 
-int launch_batch(int integ, int prec, const BatchArgs &b, int block, cudaStream_t s,
-                 double share, bool high_priority) {
+int launch_batch(int integ, int prec, const BatchArgs &b, int block, cudaStream_t s) {
   using namespace adaptive;
   if (b.nseg <= 0 || b.nseg > kMaxSegments) return kErrUnsupported;
   int64_t total = 0;
@@ -255,10 +254,9 @@ int launch_batch(int integ, int prec, const BatchArgs &b, int block, cudaStream_
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
   const int64_t full = (int64_t)std::max(1, per_sm) * sms;
-  const int64_t cap = std::max<int64_t>(1, (int64_t)(full * std::min(1.0, std::max(share, 0.0))));
-  const int64_t grid = std::min<int64_t>(cap, (total + block - 1) / block);
-  return (int)launch_with_priority(kern, (unsigned)grid, (unsigned)block, s, high_priority,
-                                  with_ctl(b, prec));
+  const int64_t grid = std::min<int64_t>(full, (total + block - 1) / block);
+  kern<<<(unsigned)grid, (unsigned)block, 0, s>>>(with_ctl(b, prec));
+  return (int)cudaGetLastError();
 }
 
 int launch_adaptive(int model, int integ, int prec, const AdaptiveArgs &a, int block, int variant,

@@ -118,9 +118,10 @@ struct chaos_lyap_handle {
   // end states of the transients, for sweeps in two launches
   void *resume = nullptr;
   int64_t resume_cap = 0;  // points
-  // second stream and fork / join events of a batch with both kernel forms
-  cudaStream_t aux_stream = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // further streams and fork / join events of a batch, one per segment after the
+  // first
+  cudaStream_t aux_stream[chaos::kMaxSegments - 1] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[chaos::kMaxSegments - 1] = {};
   // host-path staging
   double *s_params = nullptr, *s_inits = nullptr, *s_spec = nullptr, *s_tavg = nullptr;
   int32_t *s_status = nullptr;
@@ -334,12 +335,14 @@ int chaos_lyap_destroy(chaos_lyap_handle *h) {
   cudaFree(h->order);
   cudaFree(h->order_scratch);
   cudaFree(h->resume);
-  if (h->aux_stream) {
-    cudaStreamSynchronize(h->aux_stream);
-    cudaStreamDestroy(h->aux_stream);
-  }
+  for (cudaStream_t s : h->aux_stream)
+    if (s) {
+      cudaStreamSynchronize(s);
+      cudaStreamDestroy(s);
+    }
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
-  if (h->ev_join) cudaEventDestroy(h->ev_join);
+  for (cudaEvent_t e : h->ev_join)
+    if (e) cudaEventDestroy(e);
   cudaStreamDestroy(h->own_stream);
   delete h;
   return CHAOS_LYAP_OK;
@@ -692,21 +695,27 @@ int chaos_lyap_autotune_map(chaos_lyap_handle *h, int64_t P, int64_t sample,
   return autotune(h, P, n, P / n, params, inits, block_out, schedule_out);
 }
 
-// A batch runs each segment in the form of its handle's schedule: segments
-// with a split schedule in the split batch kernel, the others in the
-// one-lane batch kernel.  When both kinds are present the two persistent
-// kernels run side by side (forked onto the first handle's second stream,
-// joined before the batch ends; captured as two branches of a graph).  The
-// split kernel -- the form chosen for segments whose longest points set the
-// run's length -- is launched first and at the device's greatest priority
-// with a full machine's grid; the one-lane kernel's blocks take the SM slots
-// that its blocks free as its queues run dry.
+// A batch runs each segment in the form of its handle's schedule, one persistent
+// launch per segment, side by side: forked onto the first handle's further
+// streams, joined before the batch ends (branches of one graph when captured).
+// Each launch is its model's own sweep kernel, and where the segments fit beside
+// one another they share the SMs from the start.  Segments with a split
+// schedule -- the form chosen for segments whose longest points set the run's
+// length -- are launched first and at the device's greatest priority; the others'
+// blocks take the slots that are left or that theirs free as their queues run
+// dry.  (One kernel per form that moved its warps from segment to segment, with
+// the registers of the largest model, ran the two forms one after the other and
+// each model slower: 3 x 128^2 points, averaging times 20-80: 36.3 -> 28.5 ms.)
 struct BatchPlan {
-  chaos::BatchArgs lane, split;
-  chaos_lyap_handle *lane_h[chaos::kMaxSegments], *split_h[chaos::kMaxSegments];
-  // scratch of the longest-first ordering of each segment with per-point times
-  void *lane_scratch[chaos::kMaxSegments], *split_scratch[chaos::kMaxSegments];
-  int integ, prec, lane_block, split_block;
+  int nseg;
+  // the segments in launch order: split ones first
+  struct Part {
+    chaos::AdaptiveArgs a;
+    chaos_lyap_handle *h;
+    void *scratch;  // of the longest-first ordering, with per-point times
+    bool split;
+  } part[chaos::kMaxSegments];
+  int integ, prec;
 };
 
 // Device buffers of one segment's longest-first hand-out order.
@@ -742,6 +751,11 @@ static int build_batch(const chaos_lyap_segment *segs, int nseg, BatchPlan *plan
   int rc0 = check_segments(segs, nseg);
   if (rc0) return rc0;
   std::memset(plan, 0, sizeof *plan);
+  plan->nseg = nseg;
+  int nsplit = 0, next_split = 0;
+  for (int i = 0; i < nseg; i++) nsplit += is_split(segs[i].handle);
+  int next_lane = nsplit;
+  chaos_lyap_handle *h0 = segs[0].handle;
   for (int i = 0; i < nseg; i++) {
     const chaos_lyap_segment &sg = segs[i];
     const chaos_lyap_desc &d = sg.handle->d;
@@ -755,10 +769,10 @@ static int build_batch(const chaos_lyap_segment *segs, int nseg, BatchPlan *plan
     if (sg.P < 0 || (sg.P > 0 && (!sg.params || !sg.inits || !sg.spectrum)))
       return fail(CHAOS_LYAP_EINVAL, "segment %d: bad arrays", i);
     const bool sp = is_split(sg.handle);
-    chaos::BatchArgs &b = sp ? plan->split : plan->lane;
-    const int j = b.nseg++;
-    (sp ? plan->split_h : plan->lane_h)[j] = sg.handle;
-    chaos::AdaptiveArgs &a = b.seg[j];
+    BatchPlan::Part &part = plan->part[sp ? next_split++ : next_lane++];
+    part.h = sg.handle;
+    part.split = sp;
+    chaos::AdaptiveArgs &a = part.a;
     a.P = sg.P;
     a.k = d.k;
     a.gs = d.gs;
@@ -781,47 +795,33 @@ static int build_batch(const chaos_lyap_segment *segs, int nseg, BatchPlan *plan
     a.status = sg.status;
     a.steps = sg.steps;
     a.queue_stride = chaos::queue_stride_for(sg.P);
-    a.order = nullptr;
-    void *scratch = nullptr;
+    a.queue = h0->queue + i;  // the first handle's counters
     if (sg.t_avg_per_point && sg.P > 0) {  // longest averaging time first
       if (own) {
         a.order = own[i].order;
-        scratch = own[i].scratch;
+        part.scratch = own[i].scratch;
       } else {
         int rc = ensure_order(sg.handle, sg.P);
         if (rc) return rc;
         a.order = sg.handle->order;
-        scratch = sg.handle->order_scratch;
+        part.scratch = sg.handle->order_scratch;
       }
     }
-    (sp ? plan->split_scratch : plan->lane_scratch)[j] = scratch;
-    b.model[j] = m->id;
   }
-  chaos_lyap_handle *h0 = segs[0].handle;
-  // the first handle's counters: one-lane segments first, then split ones
-  plan->lane.queues = h0->queue;
-  plan->split.queues = h0->queue + plan->lane.nseg;
   const chaos_lyap_desc &d0 = h0->d;
   plan->integ = d0.integrator == CHAOS_INTEG_DOPRI5 ? chaos::kDopri5 : chaos::kDverk65;
   plan->prec = d0.precision == CHAOS_PREC_FP32 ? chaos::kFP32 : chaos::kFP64;
-  plan->lane_block = plan->lane.nseg ? plan->lane_h[0]->block : 128;
-  plan->split_block = plan->split.nseg ? plan->split_h[0]->block : 64;
-  if (plan->lane.nseg && plan->split.nseg && !h0->aux_stream) {  // fork / join resources
+  if (nseg > 1) {  // fork / join resources
     DeviceGuard g(d0.device);
-    cudaError_t e = cudaStreamCreateWithFlags(&h0->aux_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h0->ev_fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h0->ev_join, cudaEventDisableTiming);
-    if (e != cudaSuccess) return cuda_fail(e, "batch fork stream / events");
-  }
-  return CHAOS_LYAP_OK;
-}
-
-static int launch_orders(const chaos::BatchArgs &b, void *const *scratch, cudaStream_t s) {
-  for (int i = 0; i < b.nseg; i++) {
-    if (!b.seg[i].order) continue;
-    int rc = chaos::launch_order_longest_first(b.seg[i].t_avg_per_point, b.seg[i].P,
-                                               const_cast<int32_t *>(b.seg[i].order), scratch[i], s);
-    if (rc) return cuda_fail((cudaError_t)rc, "order launch");
+    cudaError_t e = cudaSuccess;
+    if (!h0->ev_fork) e = cudaEventCreateWithFlags(&h0->ev_fork, cudaEventDisableTiming);
+    for (int i = 0; i + 1 < nseg && e == cudaSuccess; i++) {
+      if (!h0->aux_stream[i])
+        e = cudaStreamCreateWithFlags(&h0->aux_stream[i], cudaStreamNonBlocking);
+      if (e == cudaSuccess && !h0->ev_join[i])
+        e = cudaEventCreateWithFlags(&h0->ev_join[i], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "batch fork streams / events");
   }
   return CHAOS_LYAP_OK;
 }
@@ -832,29 +832,37 @@ static int batch_rc(int rc) {
   return CHAOS_LYAP_OK;
 }
 
+static int launch_part(const BatchPlan &p, const BatchPlan::Part &q, cudaStream_t s) {
+  const chaos_lyap_handle *h = q.h;
+  if (q.split)
+    return batch_rc(chaos::launch_split(h->model->id, p.integ, p.prec, q.a, h->block, h->variant, s,
+                                        p.nseg > 1));
+  return batch_rc(chaos::launch_adaptive(h->model->id, p.integ, p.prec, q.a, h->block, h->variant, s));
+}
+
 static int enqueue_batch(const BatchPlan &p, chaos_lyap_handle *h0, cudaStream_t s) {
-  const int nseg = p.lane.nseg + p.split.nseg;
-  cudaError_t e = cudaMemsetAsync(h0->queue, 0, sizeof(unsigned long long) * nseg, s);
+  cudaError_t e = cudaMemsetAsync(h0->queue, 0, sizeof(unsigned long long) * p.nseg, s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(queues)");
-  int rc = launch_orders(p.lane, p.lane_scratch, s);
-  if (!rc) rc = launch_orders(p.split, p.split_scratch, s);
-  if (rc) return rc;
-  if (p.lane.nseg && p.split.nseg) {
-    cudaStream_t aux = h0->aux_stream;
-    if ((e = cudaEventRecord(h0->ev_fork, s)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(aux, h0->ev_fork, 0)) != cudaSuccess)
+  if (p.nseg > 1 && (e = cudaEventRecord(h0->ev_fork, s)) != cudaSuccess)
+    return cuda_fail(e, "batch fork");
+  int rc = CHAOS_LYAP_OK;
+  for (int i = 0; i < p.nseg; i++) {
+    const BatchPlan::Part &q = p.part[i];
+    const cudaStream_t t = i ? h0->aux_stream[i - 1] : s;
+    if (i && (e = cudaStreamWaitEvent(t, h0->ev_fork, 0)) != cudaSuccess)
       return cuda_fail(e, "batch fork");
-    rc = batch_rc(chaos::launch_batch_split(p.integ, p.prec, p.split, p.split_block, s, 1.0, true));
-    const int rc2 = batch_rc(chaos::launch_batch(p.integ, p.prec, p.lane, p.lane_block, aux, 1.0));
+    if (!rc && q.a.order) {
+      rc = chaos::launch_order_longest_first(q.a.t_avg_per_point, q.a.P,
+                                             const_cast<int32_t *>(q.a.order), q.scratch, t);
+      if (rc) rc = cuda_fail((cudaError_t)rc, "order launch");
+    }
+    if (!rc) rc = launch_part(p, q, t);
     // join even after a failed launch, so that a capture still ends cleanly
-    if ((e = cudaEventRecord(h0->ev_join, aux)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(s, h0->ev_join, 0)) != cudaSuccess)
+    if (i && ((e = cudaEventRecord(h0->ev_join[i - 1], t)) != cudaSuccess ||
+              (e = cudaStreamWaitEvent(s, h0->ev_join[i - 1], 0)) != cudaSuccess))
       return cuda_fail(e, "batch join");
-    return rc ? rc : rc2;
   }
-  if (p.split.nseg)
-    return batch_rc(chaos::launch_batch_split(p.integ, p.prec, p.split, p.split_block, s));
-  return batch_rc(chaos::launch_batch(p.integ, p.prec, p.lane, p.lane_block, s));
+  return rc;
 }
 
 int chaos_lyap_run_batch(const chaos_lyap_segment *segs, int nseg, void *stream) {

@@ -146,12 +146,10 @@ struct BatchArgs {
   unsigned long long *queues;      // nseg point counters, zeroed before the launch
 };
 
-// share: fraction (0, 1] of a full machine's resident blocks the persistent
-// grid may take; high_priority: launch at the device's greatest stream
-// priority (the block scheduler dispatches its pending blocks first when
-// another batch kernel runs beside it).
-int launch_batch(int integrator, int precision, const BatchArgs &b, int block, cudaStream_t s,
-                 double share = 1.0, bool high_priority = false);
+// The batch of the entry that can allocate nothing (static_scratch.cu): one
+// launch, no further streams.  (Batches of handles launch each segment's sweep
+// kernel side by side, which is faster: capi.cu.)
+int launch_batch(int integrator, int precision, const BatchArgs &b, int block, cudaStream_t s);
 
 // Kernel launch with an optional priority launch attribute (kept by stream
 // capture as the graph node's priority).
@@ -180,9 +178,7 @@ inline cudaError_t launch_with_priority(void (*kern)(Args...), unsigned grid, un
 // Split form (split.cu): one point per group of four lanes; variant 1 is the
 // exchange layout of the FP64 form for 3-dimensional models.
 int launch_split(int model, int integrator, int precision, const AdaptiveArgs &a, int block,
-                 int variant, cudaStream_t s);
-int launch_batch_split(int integrator, int precision, const BatchArgs &b, int block,
-                       cudaStream_t s, double share = 1.0, bool high_priority = false);
+                 int variant, cudaStream_t s, bool high_priority = false);
 
 }  // namespace chaos
 

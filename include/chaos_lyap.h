@@ -78,9 +78,9 @@ enum { CHAOS_LAYOUT_POINT_MAJOR = 0, CHAOS_LAYOUT_COMP_MAJOR = 1 };
  *  SPLIT_DIRECT / SPLIT_PERSISTENT: one point per group of four lanes (each
  *    lane the state and one tangent vector): about half the work per lane and
  *    step, for sweeps of few points or runs bounded by their longest point.
- *    A batch runs each segment in the form of its handle's schedule; with
- *    both forms present the two batch kernels run side by side, the split
- *    one first and at the greatest stream priority.
+ *    A batch runs each segment in the form of its handle's schedule, the
+ *    segments' launches side by side, split ones first and at the greatest
+ *    stream priority.
  *  AUTO: persistent until chaos_lyap_autotune picks one. */
 enum {
   CHAOS_SCHED_AUTO = 0,
@@ -199,8 +199,9 @@ int chaos_lyap_autotune_map(chaos_lyap_handle *h, int64_t P, int64_t sample,
 /* ---------------------------------------------------------- mixed batches
  * Several sweeps (segments: different 3- or 4-dimensional models, each with
  * its own handle, arrays and phase times; per-point averaging times allowed)
- * in ONE persistent launch whose lanes take points segment after segment, so
- * points of uneven dimension and length share warps without idling them.
+ * enqueued as one piece of work: each segment is one persistent launch of its
+ * model's sweep kernel, the segments run side by side and share the GPU, and
+ * `stream` waits for all of them.
  * All handles must use the same integrator and precision; nseg <= 8; every
  * segment has its own handle (a handle in two segments is rejected).  The
  * point counters live in the first segment's handle: do not run that handle
