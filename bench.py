@@ -206,11 +206,12 @@ def cpu_reference(w, params, inits, sample, threads, seed=0):
     import oracle
     rng = np.random.default_rng(seed)
     idx = rng.choice(params.shape[0], sample, replace=False)
+    # without the reference's sources: the oracle's restatement of them
+    fixed = oracle.reference if oracle.have_ref() else oracle.fixed
     t0 = time.perf_counter()
-    out, _ = oracle.reference(w["model"], "var", params[idx], inits[idx], 1e-7, w["ref_h"],
-                              w.get("k", 3),
-                              w["t_transient"], 0.0, w["t_avg"], w["dt_renorm"] / w["ref_h"],
-                              threads=threads)
+    out, _ = fixed(w["model"], "var", params[idx], inits[idx], 1e-7, w["ref_h"], w.get("k", 3),
+                   w["t_transient"], 0.0, w["t_avg"], w["dt_renorm"] / w["ref_h"],
+                   threads=threads)
     dt = time.perf_counter() - t0
     return sample / dt, dt, idx, out
 
@@ -234,6 +235,11 @@ def run_reference_arm(a, w, rank):
         return
     threads = os.cpu_count() or 1
     import oracle
+    if not oracle.have_ref():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's sources are not here: oracle/_ref "
+                                         "could not be built"}), flush=True)
+        return
     params, inits = build_inputs(w, 0, src=oracle)
     # per step about 20 s of the host's threads
     sample = int(max(threads, min(4096, 20.0 * threads / ref_seconds_per_point(w))))
@@ -529,11 +535,12 @@ def measure_batch(a, rank, world, local, nsteps, nwarm, unbatched=True):
                    "t_avg": (f"U[1000, 10000] x {a.t_scale:g} per point" if a.t_scale != 1.0
                              else "U[1000, 10000] per point"),
                    **{k: v for k, v in BATCH_KW.items() if k != "t_avg"},
-                   "launch": "one persistent batch kernel per step, replayed CUDA graph",
+                   "launch": "one sweep kernel per segment, side by side, replayed CUDA graph",
                    "form": {name: ("one point per group of four lanes"
                                    if form_of(name).startswith("split") else
                                    "one point per lane") for name in BATCH}},
-        "gpu_launches": nsteps, "clocks": clk,
+        # per segment: four kernels of the longest-first order and the sweep
+        "gpu_launches": nsteps * 5 * len(BATCH), "clocks": clk,
         "roofline": {"bound": "fp32_fma", "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                      "peak_source": "measured in-process (FMA-chain kernel)"},
@@ -849,7 +856,10 @@ def run_sweep_bench(a, w, rank, world, local):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": w["dtype"], "data": "synthetic (seeded grid and jitter)",
         "config": config_of(a, w, extra={"launch": tuned}),
-        "gpu_launches": a.steps,
+        # persistent sweeps of more than 1.5 waves: the transients, four kernels of
+        # the longest-first order and the averaging phases; otherwise one kernel
+        "gpu_launches": a.steps * (6 if tuned.get("schedule") == "persistent" and P >= 120_000
+                                   else 1),
         "clocks": clk,
         "roofline": {"bound": "fp32_fma" if w["precision"] == "fp32" else "fp64_fma",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",

@@ -392,9 +392,10 @@ constexpr int64_t kTwoPhaseMaxWaves = 32;
 static int ensure_resume(chaos_lyap_handle *h, int64_t P, cudaStream_t s, bool *ready) {
   *ready = false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(s, &cap);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
-  if (cap != cudaStreamCaptureStatusNone) return CHAOS_LYAP_OK;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return CHAOS_LYAP_OK;
+  }
   if (P > h->resume_cap) {
     DeviceGuard g(h->d.device);
     cudaFree(h->resume);
