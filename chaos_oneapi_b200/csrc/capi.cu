@@ -8,6 +8,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 
 #include "../../include/chaos_lyap.h"
@@ -101,6 +103,51 @@ int model_id_of(const char *name, int *dim, int *nparams) {
 }
 }  // namespace chaos
 
+// Memory of the two-launch sweeps (see TwoPhase): one pool per device, made with
+// the device's first adaptive handle and destroyed with its last, shared by all
+// of them in stream order.  It keeps at most kPoolKeepBytes between runs (the
+// rest goes back at the next synchronisation).  cudaMalloc inside a new
+// handle's first run took 0.5-16 ms on a shared host.
+struct ResumePool {
+  cudaMemPool_t pool = nullptr;
+  int handles = 0;
+};
+constexpr uint64_t kPoolKeepBytes = 256ull << 20;
+static std::mutex g_pool_mutex;
+// never destroyed: handles may outlive static destruction
+static std::map<int, ResumePool> &g_pools = *new std::map<int, ResumePool>;
+
+// nullptr if the device has no memory pools: its sweeps run as one launch.
+static cudaMemPool_t pool_acquire(int device) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  ResumePool &p = g_pools[device];
+  if (!p.pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&p.pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      p.pool = nullptr;
+      return nullptr;
+    }
+    uint64_t keep = kPoolKeepBytes;
+    int off = 0;  // another stream's block only once its work is done: sweeps on two streams overlap
+    cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaMemPoolSetAttribute(p.pool, cudaMemPoolReuseAllowInternalDependencies, &off);
+  }
+  ++p.handles;
+  return p.pool;
+}
+
+static void pool_release(int device) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  ResumePool &p = g_pools[device];
+  if (--p.handles > 0) return;
+  cudaMemPoolDestroy(p.pool);
+  p.pool = nullptr;
+}
+
 struct chaos_lyap_handle {
   chaos_lyap_desc d;
   const ModelInfo *model;
@@ -115,9 +162,7 @@ struct chaos_lyap_handle {
   int32_t *order = nullptr;
   void *order_scratch = nullptr;
   int64_t order_cap = 0;
-  // end states of the transients, for sweeps in two launches
-  void *resume = nullptr;
-  int64_t resume_cap = 0;  // points
+  cudaMemPool_t pool = nullptr;  // the device's ResumePool, if this handle holds it
   // further streams and fork / join events of a batch, one per segment after the
   // first
   cudaStream_t aux_stream[chaos::kMaxSegments - 1] = {};
@@ -309,6 +354,7 @@ int chaos_lyap_create(const chaos_lyap_desc *desc, chaos_lyap_handle **out) {
     delete h;
     return fail(CHAOS_LYAP_ENOMEM, "cudaMalloc(queue): %s", cudaGetErrorString(e));
   }
+  if (d.precision != CHAOS_PREC_COMPAT_FP64) h->pool = pool_acquire(d.device);
   *out = h;
   return CHAOS_LYAP_OK;
 }
@@ -334,7 +380,7 @@ int chaos_lyap_destroy(chaos_lyap_handle *h) {
   cudaFree(h->queue);
   cudaFree(h->order);
   cudaFree(h->order_scratch);
-  cudaFree(h->resume);
+  if (h->pool) pool_release(h->d.device);
   for (cudaStream_t s : h->aux_stream)
     if (s) {
       cudaStreamSynchronize(s);
@@ -373,9 +419,9 @@ static int ensure_order(chaos_lyap_handle *h, int64_t P) {
 // the order cannot matter; just above one wave the run is its longest points
 // either way) but few enough waves that the end of the run, where lanes wait
 // for the longest points started last, is a sizeable part of it.  Needs a
-// transient (it is what predicts the cost); the buffers, 48-76 bytes per point
-// (Lorenz-96: 344), are kept by the handle.  One launch -> two, B200: 256^2 Lorenz points in FP64
-// (1.7 waves) 245 -> 195 ms; FP32 Lorenz, 152k points (2 waves) 62 -> 47 ms,
+// transient (it is what predicts the cost); the buffers take 48-92 bytes per
+// point (Lorenz-96: 344-668).  One launch -> two, B200: 256^2 Lorenz points in
+// FP64 (1.7 waves) 245 -> 195 ms; FP32 Lorenz, 152k points (2 waves) 62 -> 47 ms,
 // 300k 103 -> 85 ms, 1024^2 (14 waves) 309 -> 275 ms; FP32 Rossler, whose
 // longest points take twice the mean, 152k points 82 -> 77 ms; at 1.1 waves of
 // it 55 -> 52 ms.
@@ -386,34 +432,43 @@ constexpr double kTwoPhaseMinWaves = 1.5;
 constexpr double kTwoPhaseMinWavesWarp = 1.0;
 constexpr int64_t kTwoPhaseMaxWaves = 32;
 
-// Buffers of a two-launch sweep of P points; *ready false during a stream
-// capture (a replay must not depend on buffers that a later run of the handle
-// may grow) or when memory is short: the sweep then runs as one launch.
-static int ensure_resume(chaos_lyap_handle *h, int64_t P, cudaStream_t s, bool *ready) {
-  *ready = false;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return CHAOS_LYAP_OK;
-  }
-  if (P > h->resume_cap) {
-    DeviceGuard g(h->d.device);
-    cudaFree(h->resume);
-    h->resume = nullptr;
-    h->resume_cap = 0;
-    const int prec = h->d.precision == CHAOS_PREC_FP32 ? chaos::kFP32 : chaos::kFP64;
-    if (cudaMalloc(&h->resume, (chaos::resume_state_bytes(h->model->dim, prec) + 16) * P) !=
+// Buffers of one two-launch sweep of P points, from the pool and back to it in
+// the order of stream s.  Empty (the sweep runs as one launch) during a stream
+// capture, where the allocation would be the graph's, and when memory is short.
+struct TwoPhase {
+  char *base = nullptr;
+  cudaStream_t s;
+  void *scratch = nullptr;
+  int32_t *order = nullptr;
+  chaos::Resume resume{};
+  TwoPhase(const chaos_lyap_handle *h, int prec, int64_t P, cudaStream_t stream) : s(stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!h->pool || cudaStreamIsCapturing(s, &cap) != cudaSuccess ||
+        cap != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return;
+    }
+    const size_t head = (chaos::kOrderScratchBytes + 255) / 256 * 256;
+    const size_t state = (size_t)chaos::resume_state_bytes(h->model->dim, prec) * P;
+    void *b = nullptr;
+    if (cudaMallocFromPoolAsync(&b, head + 16 * P + state + sizeof(int32_t) * P, h->pool, s) !=
         cudaSuccess) {
       cudaGetLastError();
-      h->resume = nullptr;
-      return CHAOS_LYAP_OK;
+      return;
     }
-    h->resume_cap = P;
+    base = static_cast<char *>(b);
+    scratch = base;
+    resume.cost = reinterpret_cast<double *>(base + head);
+    resume.steps = reinterpret_cast<int64_t *>(resume.cost + P);
+    resume.state = resume.steps + P;
+    order = reinterpret_cast<int32_t *>(base + head + 16 * P + state);
   }
-  *ready = ensure_order(h, P) == CHAOS_LYAP_OK;
-  if (!*ready) cudaGetLastError();
-  return CHAOS_LYAP_OK;
-}
+  ~TwoPhase() {
+    if (base) cudaFreeAsync(base, s);
+  }
+  TwoPhase(const TwoPhase &) = delete;
+  TwoPhase &operator=(const TwoPhase &) = delete;
+};
 
 // P points of params / inits are read at every `stride`-th point of arrays
 // that hold P_full points (stride 1, P_full = 0: the arrays themselves); the
@@ -475,31 +530,29 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
       if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(queue)");
       a.queue = h->queue;
       a.queue_stride = chaos::queue_stride_for(P);
-      bool two_phase = false;
       const bool warp = m->dim > 4;
       if (!split && a.t_transient > 0) {
         const int64_t held = warp ? chaos::l96_resident(integ, prec, d.k)
                                   : chaos::adaptive_resident(m->id, integ, prec, block, variant);
         const double least = warp ? kTwoPhaseMinWavesWarp : kTwoPhaseMinWaves;
-        if (held > 0 && P > (int64_t)(least * held) && P <= kTwoPhaseMaxWaves * held &&
-            (rc = ensure_resume(h, P, s, &two_phase)))
-          return rc;
-      }
-      if (two_phase) {
-        a.order = h->order;
-        a.resume.cost = static_cast<double *>(h->resume);
-        a.resume.steps = reinterpret_cast<int64_t *>(a.resume.cost + P);
-        a.resume.state = a.resume.steps + P;
-        rc = warp ? chaos::launch_l96_two_phase(integ, prec, a, h->order_scratch, s)
-                  : chaos::launch_adaptive_two_phase(m->id, integ, prec, a, block, variant,
-                                                     h->order_scratch, s);
-        if (rc && rc != chaos::kErrUnsupported) return cuda_fail((cudaError_t)rc, "kernel launch");
-        if (!rc) {
-          h->last_stream = s;
-          return CHAOS_LYAP_OK;
+        if (held > 0 && P > (int64_t)(least * held) && P <= kTwoPhaseMaxWaves * held) {
+          TwoPhase t(h, prec, P, s);
+          if (t.base) {
+            a.order = t.order;
+            a.resume = t.resume;
+            rc = warp ? chaos::launch_l96_two_phase(integ, prec, a, t.scratch, s)
+                      : chaos::launch_adaptive_two_phase(m->id, integ, prec, a, block, variant,
+                                                         t.scratch, s);
+            if (rc && rc != chaos::kErrUnsupported)
+              return cuda_fail((cudaError_t)rc, "kernel launch");
+            if (!rc) {
+              h->last_stream = s;
+              return CHAOS_LYAP_OK;
+            }
+            a.resume = chaos::Resume{};
+            a.order = nullptr;
+          }
         }
-        a.resume = chaos::Resume{};
-        a.order = nullptr;
       }
       if (a.t_avg_per_point && m->dim <= 4) {  // longest averaging time first
         if ((rc = ensure_order(h, P))) return rc;

@@ -98,3 +98,37 @@ def test_two_launches_with_own_averaging_times_and_capture(lib):
     one, st1, _ = _run(lib, torch, p, x, "point", 20_000, **kw)
     assert np.array_equal(status, st1)
     assert np.abs(spec[ok] - one[ok]).max() < 1e3 * RTOL
+
+
+def test_sweeps_share_their_memory_across_handles_and_streams(lib):
+    """Handles on streams of their own, made and closed while others run: each
+    sweep has its own buffers until its last kernel is done."""
+    import torch
+    P = 60_001
+    sets = [_inputs(P, seed) for seed in (11, 12, 13)]
+    kw = dict(precision="fp64", integrator="dopri5")
+    want = [_run(lib, torch, p, x, "point", 20_000, **kw) for p, x in sets]
+    live, got = [], []
+    for i in (0, 1, 2, 0, 1):
+        p, x = (torch.from_numpy(a).cuda() for a in sets[i])
+        ds = torch.zeros((P, 3), dtype=torch.float64, device="cuda")
+        st = torch.full((P,), -1, dtype=torch.int32, device="cuda")
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        sw = lib.Sweep(model="lorenz", method="var", rtol=RTOL, atol=RTOL, h=1e-3,
+                       t_transient=2.0, t_avg=6.0, dt_renorm=1.0, layout="point",
+                       schedule="persistent", **kw)
+        with torch.cuda.stream(s):
+            sw.run(p, x, ds, st, None, stream=s.cuda_stream)
+        live.append(sw)
+        got.append((i, p, x, ds, st, s))
+        if len(live) == 4:
+            live.pop(0).close()
+    torch.cuda.synchronize()
+    for sw in live:
+        sw.close()
+    for i, _, _, ds, st, _ in got:
+        spec, status, _ = want[i]
+        ok = status == 0
+        assert np.array_equal(st.cpu().numpy(), status)
+        assert np.abs(ds.cpu().numpy()[ok] - spec[ok]).max() < 1e3 * RTOL
