@@ -5,7 +5,9 @@
 //    SM count) whose threads pull point indices from a device counter, so a
 //    thread whose point needed fewer adaptive steps (or a shorter averaging
 //    time) starts the next point at once instead of idling until the
-//    slowest lane of its warp is done.
+//    slowest lane of its warp is done.  A sweep of a few waves runs as two
+//    such launches, every point's transient, then the averaging phases
+//    longest first (launch_adaptive_two_phase).
 #include <algorithm>
 
 #include "adaptive.cuh"

@@ -1,6 +1,7 @@
 // Learned surrogate: an ensemble of small MLPs mapping a parameter point
 // (p1, p2) to its Lyapunov spectrum, trained and evaluated on the GPU by the
-// kernels below (no library GEMM).
+// kernels below (no library GEMM); widths 64 and 128 take the fused kernels
+// of mlp_fused.cu.
 //
 //   features: 16 Fourier features of the point normalised to [0, 1]^2:
 //             sin / cos (2 pi w_f . (u, v)) for 8 frequency vectors (default
