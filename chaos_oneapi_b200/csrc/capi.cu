@@ -8,7 +8,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <string>
 
@@ -114,11 +113,12 @@ struct ResumePool {
 };
 constexpr uint64_t kPoolKeepBytes = 256ull << 20;
 static std::mutex g_pool_mutex;
-// never destroyed: handles may outlive static destruction
-static std::map<int, ResumePool> &g_pools = *new std::map<int, ResumePool>;
+constexpr int kPoolDevices = 64;
+static ResumePool g_pools[kPoolDevices];
 
 // nullptr if the device has no memory pools: its sweeps run as one launch.
 static cudaMemPool_t pool_acquire(int device) {
+  if (device >= kPoolDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   ResumePool &p = g_pools[device];
   if (!p.pool) {
