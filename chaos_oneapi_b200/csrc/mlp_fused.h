@@ -107,22 +107,24 @@ __device__ __forceinline__ float dsilu(float z) {
   return sg * (1.f + z * (1.f - sg));
 }
 
-// z / d for 1 <= d < kFastDivLimit: a reciprocal refined by Newton's method,
-// then Markstein's quotient correction (IBM J. Res. Dev. 34, 1990, 111-119),
-// which leaves the correctly rounded quotient.  The general division takes a
-// third special-function operation per element (its operand check) and a
-// branch; the fused epilogues are bound by that unit.  The callers send a
-// chunk with a larger d (SiLU at z < -85) through the general division.
+// z / d for finite z and 1 <= d < kFastDivLimit: an approximate reciprocal
+// refined by one step of Newton's method, then Markstein's quotient correction
+// (IBM J. Res. Dev. 34, 1990, 111-119).  Equal to the `/` operator, signed zeros
+// included, for every z with d = 1 + e^-z and for z = 1 with every d of the range
+// (tests/test_gpu_silu.py runs all of them).  The fused epilogues are bound by
+// the special-function pipe (71 % busy in predict_kernel), which this uses once
+// per quotient.  The callers send a chunk with a larger d (SiLU at z < -85), a
+// NaN or an infinite z through the plain functions.
 constexpr float kFastDivLimit = 1e37f;
 __device__ __forceinline__ float divide_above_one(float z, float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   r = fmaf(fmaf(-d, r, 1.f), r, r);
   const float q = z * r;
-  return fmaf(fmaf(-q, d, z), r, q);
+  return fmaf(-fmaf(q, d, -z), r, q);  // (the remainder negated twice keeps -0)
 }
 // 1 + e^-z as 1 + 2^(-z log2 e).  Denormal powers may flush to zero: the sum is
-// 1 either way, and the instruction needs no scaling around it.
+// 1 either way.
 __device__ __forceinline__ float one_plus_exp_neg(float z) {
   float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-z * 1.44269504088896341f));
@@ -135,7 +137,11 @@ template <int N> __device__ __forceinline__ void silu_chunk(float (&v)[N]) {
 #pragma unroll
   for (int i = 0; i < N; i++) {
     const float d = one_plus_exp_neg(v[i]);
-    fast = fast && d < kFastDivLimit;  // false for NaN
+    // false for NaN; at z = +inf the quotient's remainder would be inf - inf.  (A
+    // second comparison per unit: 2^20 rows of 4 networks of width 128 take 1.119
+    // ms instead of 1.116; a maximum over the chunk, or z x 0 added to d, 1.143 and
+    // 1.160.)
+    fast = fast && d < kFastDivLimit && v[i] < INFINITY;
     q[i] = divide_above_one(v[i], d);
   }
   if (fast) {
