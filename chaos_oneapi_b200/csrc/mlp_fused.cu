@@ -333,17 +333,18 @@ __global__ void __launch_bounds__(kTrainThreads, 1) train_kernel(const __grid_co
       }
     }
   }
-  wait_previous();
-  launch_dependents();
-  if (tid == 0) load_weights<W>(g, z, base, wbar);
-  load_biases<W>(g, z, bias);
-  if (z == 0)
-    *reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(g.b.X) +
-                                  ((fi >> 3) * 2 + (fh >> 2)) * 128 + fin) = fq;
+  // (launch_dependents only once this CTA holds its tensor memory: umma.cuh)
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = *slot;
+  wait_previous();
+  launch_dependents();
+  if (tid == 0) load_weights<W>(g, z, base, wbar);
+  load_biases<W>(g, z, bias);  // read after the first product's barrier
+  if (z == 0)
+    *reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(g.b.X) +
+                                  ((fi >> 3) * 2 + (fh >> 2)) * 128 + fin) = fq;
   const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
   Product product{mbar, 0, mbar_wait(wbar, 0)};
   const int64_t row0 = z * padded + tile * kTrainRows;  // the tile's first row in the buffers
@@ -540,12 +541,12 @@ __device__ void weight_gradient(const GradArgs &g, int l, int n0, int z, uint8_t
     mo = read(g.P.m, tid);
     ve = read(g.P.v, tid);
   }
-  wait_previous();
-  launch_dependents();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = *slot;
+  wait_previous();
+  launch_dependents();
   int *flag = reinterpret_cast<int *>(slot + 1);
   if (warp == 1) {  // loads, one copy per lane
     bool ok = true;

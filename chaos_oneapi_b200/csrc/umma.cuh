@@ -77,7 +77,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 // Programmatic dependent launch: the next kernel of the stream may start its
 // preamble once every block of this one has called launch_dependents; its
 // wait_previous returns when this kernel has finished and its writes are
-// visible.  (Both do nothing in a kernel launched without the attribute.)
+// visible.  (Both do nothing in a kernel launched without the attribute.)  A CTA
+// calls launch_dependents only once it holds its tensor memory: a dependent's CTA
+// takes columns of its own and keeps them while it waits for this kernel, which
+// must not still be waiting for those columns.
 __device__ __forceinline__ void launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
