@@ -436,6 +436,16 @@ constexpr int64_t kTwoPhaseMaxWaves = 32;
 // the order of stream s.  Empty (the sweep runs as one launch) during a stream
 // capture, where the allocation would be the graph's, and when memory is short.
 struct TwoPhase {
+  // An allocation from the pool is refused, and ends the capture, while a capture
+  // of another stream is open (this thread's, or a global one of any thread's),
+  // unless the calling thread's mode is relaxed.  Nothing below depends on what a
+  // capture of another stream records, so it is.  (Restored last: the block goes
+  // back to the pool under it.)
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
   char *base = nullptr;
   cudaStream_t s;
   void *scratch = nullptr;
