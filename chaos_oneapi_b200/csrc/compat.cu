@@ -15,6 +15,9 @@
 //     length eps: cuda/tools/linalg.dp.cpp:20-51; QR by column CGS and
 //     R = Q^T A: :54-127 (square case).
 // This translation unit must be compiled with -fmad=false.
+#include <type_traits>
+
+#include "compat_rule.h"
 #include "kernels.h"
 #include "models.cuh"
 
@@ -365,7 +368,7 @@ __global__ void __launch_bounds__(128) compat_kernel(const CompatArgs a) {
 // run beside each other.  Every row goes through the operations of the
 // one-thread form in their order (no multiply-add is contracted here): the same
 // bits.  The price is the state-only phase, which every lane repeats, and a
-// right-hand side evaluated for both kinds of row; see kMaxLanePointsPerSm.
+// right-hand side evaluated for both kinds of row; see compat_rule.h.
 template <int N> struct Rows {
   int i;          // vector index, < 0: the state
   int base;       // the group's first lane
@@ -542,24 +545,17 @@ __global__ void __launch_bounds__(32) compat_rows_kernel(const CompatArgs a) {
   if (a.status && r == 0) a.status[pt] = finite ? 0 : 1;
 }
 
-// Up to this many points per SM a group of lanes per point is faster than a
-// thread.  One thread per point is one row's latency times 1 + k until its
-// threads fill the schedulers (16,384 points: one warp each); the groups are
-// bound by the FP64 pipe from about 30 points per SM on.  800 steps, k = 3, one
-// thread / group: Shimizu FD 1,024 points 967 / 328 us, 7,680 points 973 / 523,
-// 12,288 points 975 / 737, 16,384 points 976 / 958, 25,600 points 1464 / 1384;
-// Lorenz QR 1,024 points 1386 / 654 us, 12,288 points 1390 / 1168, 16,384 points
-// 1391 / 1474; Lorenz VAR 12,288 points 1028 / 863, 16,384 points 1028 / 1120.
-constexpr int64_t kMaxLanePointsPerSm = 88;
-
 template <class M, int KT>
 int launch_one(const CompatArgs &a, int block, cudaStream_t s) {
   if constexpr (KT > 0 && !IsMap<M>::value) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (a.P <= kMaxLanePointsPerSm * sms && (a.method != 2 || KT == M::N)) {
-      constexpr int G = KT + 1 <= 2 ? 2 : KT + 1 <= 4 ? 4 : 8;
+    constexpr bool chua = std::is_same<M, Chua>::value;
+    const CompatSteps n =
+        compat_steps(a.method, a.step, a.t_skip, a.t_skip_clp, a.calc_time, a.add_skip);
+    if ((a.method != 2 || KT == M::N) && compat_rows_faster(a.method, KT, chua, a.P, sms, n)) {
+      constexpr int G = compat_row_lanes(KT);
       const int64_t grid = (a.P + 32 / G - 1) / (32 / G);
       compat_rows_kernel<M, KT, G><<<(unsigned)grid, 32, 0, s>>>(a);
       return (int)cudaGetLastError();
