@@ -50,8 +50,8 @@ __device__ __forceinline__ void lane_begin(Lane<M, K, R, INTEG> &L, const Adapti
 // is voted per warp: when any lane is due, every lane past its transient
 // renormalises in the same pass.
 // MINB: resident 128-thread blocks per SM the kernel is compiled for (a
-// register cap: 4 -> 128 registers, 5 -> 96 with a few spills); the
-// autotuner picks the variant.
+// register cap: 3 -> 168 registers, 4 -> 128, 5 -> 96 with a few spills); the
+// autotuner picks the variant, except in batches (kBatchVariant).
 // RESUME: the averaging phases of points whose transients have run.
 template <class M, int K, class R, int INTEG, int MINB, bool RESUME = false>
 __global__ void __launch_bounds__(128, MINB) sweep_kernel(const AdaptiveArgs a) {
@@ -87,11 +87,14 @@ __global__ void __launch_bounds__(128) transient_kernel(const AdaptiveArgs a) {
 }
 
 template <class M, class R, int INTEG, bool RESUME> auto sweep_kernel_of(int variant) {
-  if constexpr (sizeof(R) == 4)
+  if constexpr (sizeof(R) == 4) {
+    if constexpr (!RESUME)  // (batches have no launch of averaging phases alone)
+      if (variant == kBatchVariant) return sweep_kernel<M, M::N, R, INTEG, 3>;
     return variant == 1 ? sweep_kernel<M, M::N, R, INTEG, 5, RESUME>
                         : sweep_kernel<M, M::N, R, INTEG, 4, RESUME>;
-  else
+  } else {
     return sweep_kernel<M, M::N, R, INTEG, 1, RESUME>;
+  }
 }
 
 // What a launch of one (model, precision, integrator) does.
@@ -99,15 +102,17 @@ struct Launch {
   enum Kind { kRun, kTransients, kAveraging, kResident } kind;
   int block, variant;
   cudaStream_t s;
-  int64_t resident;  // result of kResident: points
+  int64_t resident;   // result of kResident: points
+  int lanes_per_sm;   // kRun: at most so many (0: all that fit)
 };
 
 // One full wave of blocks: resident blocks per SM x SM count.
-template <class K> int64_t full_wave(K kern, int block) {
+template <class K> int64_t full_wave(K kern, int block, int lanes_per_sm = 0) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
+  if (lanes_per_sm > 0) per_sm = std::min(per_sm, lanes_per_sm / block);
   return (int64_t)std::max(1, per_sm) * std::max(1, sms);
 }
 
@@ -132,7 +137,8 @@ template <class M, class R, int INTEG> int launch_mri(const AdaptiveArgs &a, Lau
     const int64_t wave = a.P < 3 * most * l.block ? std::min(most, base) : most;
     resume<<<(unsigned)std::min(wave, need), l.block, 0, l.s>>>(ka);
   } else {
-    const int64_t grid = a.queue ? std::min(full_wave(kern, l.block), need) : need;
+    const int64_t grid =
+        a.queue ? std::min(full_wave(kern, l.block, l.lanes_per_sm), need) : need;
     kern<<<(unsigned)grid, l.block, 0, l.s>>>(ka);
   }
   return (int)cudaGetLastError();
@@ -262,16 +268,16 @@ int launch_batch(int integ, int prec, const BatchArgs &b, int block, cudaStream_
 }
 
 int launch_adaptive(int model, int integ, int prec, const AdaptiveArgs &a, int block, int variant,
-                    cudaStream_t s) {
+                    cudaStream_t s, int lanes_per_sm) {
   using namespace adaptive;
   if (a.P <= 0) return 0;
-  Launch l{Launch::kRun, block, variant, s, 0};
+  Launch l{Launch::kRun, block, variant, s, 0, lanes_per_sm};
   return launch_model(model, integ, prec, a, l);
 }
 
 int64_t adaptive_resident(int model, int integ, int prec, int block, int variant) {
   using namespace adaptive;
-  Launch l{Launch::kResident, block, variant, nullptr, 0};
+  Launch l{Launch::kResident, block, variant, nullptr, 0, 0};
   return launch_model(model, integ, prec, AdaptiveArgs{}, l) ? 0 : l.resident;
 }
 
@@ -279,7 +285,7 @@ int launch_adaptive_two_phase(int model, int integ, int prec, const AdaptiveArgs
                               int variant, void *order_scratch, cudaStream_t s) {
   using namespace adaptive;
   if (a.P <= 0) return 0;
-  Launch l{Launch::kTransients, block, variant, s, 0};
+  Launch l{Launch::kTransients, block, variant, s, 0, 0};
   int rc = launch_model(model, integ, prec, a, l);
   if (!rc)
     rc = launch_order_longest_first(a.resume.cost, a.P, const_cast<int32_t *>(a.order),

@@ -769,7 +769,37 @@ int chaos_lyap_autotune_map(chaos_lyap_handle *h, int64_t P, int64_t sample,
 // blocks take the slots that are left or that theirs free as their queues run
 // dry.  (One kernel per form that moved its warps from segment to segment, with
 // the registers of the largest model, ran the two forms one after the other and
-// each model slower: 3 x 128^2 points, averaging times 20-80: 36.3 -> 28.5 ms.)
+// each model slower.)
+//
+// An FP32 batch of few waves whose points have averaging times of their own is as
+// long as its longest points' chains of steps, and a step takes longer the more
+// warps share its scheduler: its one-lane segments run in the build of three
+// blocks per SM instead of four, whichever segments share an SM.  Averaging times T
+// to 4 T, one kernel for all / four blocks / three: 65,536 hyper-Rossler and 65,536
+// Lorenz points 307 / 371 / 305 ms, with as many Chua points 383 / 391 / 298 ms;
+// 150,000 Lorenz points (2 waves) 8.0 / 6.8 / 6.8 ms.  From kBatchFewWaves waves of
+// the four-block build on its throughput counts: 300,000 Lorenz points (4 waves)
+// 15.2 / 12.3 / 12.9 ms.  Segments that lie apart gain nothing: 19,891 Lorenz and as
+// many Rossler points (0.5 waves) 4.1 / 3.0-3.3 / 3.3 ms, eight segments of 4,096
+// 3.6 / 1.4 / 1.5 ms; beside a split segment they meet sooner (3 x 128^2 points, 0.4
+// waves of them: 36.1 / 27.8 / 26.5 ms).
+constexpr double kBatchFewWaves = 3.0, kBatchApartWaves = 0.6, kBatchApartWavesSplit = 0.25;
+// Such a batch of one segment takes two blocks per SM while its points come out
+// even over them: up to kBatchSoloWaves times the build's lanes.  One kernel / four
+// blocks / three / two: hyper-Rossler, 39,782 points 252 / 278 / 294 / 223 ms, 65,546
+// points 280 / 384 / 297 / 221, 77,670 points 291 / 387 / 299 / 227; Lorenz, 39,782
+// points 3.5 / 4.0 / 3.9 / 3.0, 77,670 points 4.6 / 5.2 / 4.1 / 4.1, 100,000 points 5.6
+// / 5.4 / 4.7 / 5.2 ms.
+constexpr int kBatchSoloLanes = 256;  // per SM
+constexpr double kBatchSoloWaves = 1.5;
+// Among the one-lane segments those of fewer points are launched first: they
+// start whole beside a part of the larger ones, whose other points follow as
+// lanes become free.  If they do not all fit, the orders are made before the
+// fork, so that the sweep kernels themselves start in that order: 120,000 Lorenz
+// and 3,000 hyper-Rossler points, either way round, 42 ms as one kernel, 27 ms
+// this way, 35 ms with the Lorenz points first; 20,000 points each of three
+// models and 5,000 of a fourth 51 ms, 27 ms, and 28-45 ms where the order was
+// left to the streams.
 struct BatchPlan {
   int nseg;
   // the segments in launch order: split ones first
@@ -780,7 +810,29 @@ struct BatchPlan {
     bool split;
   } part[chaos::kMaxSegments];
   int integ, prec;
+  bool few_waves;    // FP32: kBatchVariant for one-lane segments of uneven points
+  bool solo;         // FP32, one such segment: kBatchSoloLanes
+  bool order_first;  // all hand-out orders before the fork
 };
+
+static int part_variant(const BatchPlan &p, const BatchPlan::Part &q) {
+  return p.few_waves && q.a.order ? chaos::kBatchVariant : q.h->variant;
+}
+
+// Points of the one-lane segments in waves of the points the GPU holds (FP32: of
+// kBatchVariant, or of the handles' builds).
+static double lane_waves(const BatchPlan &p, bool batch_build) {
+  double waves = 0;
+  for (int i = 0; i < p.nseg; i++) {
+    const BatchPlan::Part &q = p.part[i];
+    if (q.split) continue;
+    const int64_t held =
+        chaos::adaptive_resident(q.h->model->id, p.integ, p.prec, q.h->block,
+                                 batch_build ? chaos::kBatchVariant : q.h->variant);
+    waves += (double)q.a.P / (double)std::max<int64_t>(1, held);
+  }
+  return waves;
+}
 
 // Device buffers of one segment's longest-first hand-out order.
 struct OrderBuf {
@@ -875,8 +927,17 @@ static int build_batch(const chaos_lyap_segment *segs, int nseg, BatchPlan *plan
   const chaos_lyap_desc &d0 = h0->d;
   plan->integ = d0.integrator == CHAOS_INTEG_DOPRI5 ? chaos::kDopri5 : chaos::kDverk65;
   plan->prec = d0.precision == CHAOS_PREC_FP32 ? chaos::kFP32 : chaos::kFP64;
+  std::stable_sort(plan->part + nsplit, plan->part + nseg,
+                   [](const BatchPlan::Part &x, const BatchPlan::Part &y) { return x.a.P < y.a.P; });
+  DeviceGuard g(d0.device);
+  const double waves = lane_waves(*plan, false);
+  plan->few_waves =
+      plan->prec == chaos::kFP32 && waves < kBatchFewWaves &&
+      (nseg == 1 || waves > (nsplit ? kBatchApartWavesSplit : kBatchApartWaves));
+  plan->solo = plan->few_waves && nseg == 1 && nsplit == 0 && plan->part[0].a.order &&
+               lane_waves(*plan, true) <= kBatchSoloWaves;
+  plan->order_first = nseg > 1 && nsplit == 0 && lane_waves(*plan, plan->few_waves) > 1.0;
   if (nseg > 1) {  // fork / join resources
-    DeviceGuard g(d0.device);
     cudaError_t e = cudaSuccess;
     if (!h0->ev_fork) e = cudaEventCreateWithFlags(&h0->ev_fork, cudaEventDisableTiming);
     for (int i = 0; i + 1 < nseg && e == cudaSuccess; i++) {
@@ -901,25 +962,30 @@ static int launch_part(const BatchPlan &p, const BatchPlan::Part &q, cudaStream_
   if (q.split)
     return batch_rc(chaos::launch_split(h->model->id, p.integ, p.prec, q.a, h->block, h->variant, s,
                                         p.nseg > 1));
-  return batch_rc(chaos::launch_adaptive(h->model->id, p.integ, p.prec, q.a, h->block, h->variant, s));
+  return batch_rc(chaos::launch_adaptive(h->model->id, p.integ, p.prec, q.a, h->block,
+                                         part_variant(p, q), s, p.solo ? kBatchSoloLanes : 0));
+}
+
+static int launch_order(const BatchPlan::Part &q, cudaStream_t s) {
+  if (!q.a.order) return CHAOS_LYAP_OK;
+  const int rc = chaos::launch_order_longest_first(q.a.t_avg_per_point, q.a.P,
+                                                   const_cast<int32_t *>(q.a.order), q.scratch, s);
+  return rc ? cuda_fail((cudaError_t)rc, "order launch") : CHAOS_LYAP_OK;
 }
 
 static int enqueue_batch(const BatchPlan &p, chaos_lyap_handle *h0, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(h0->queue, 0, sizeof(unsigned long long) * p.nseg, s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(queues)");
+  int rc = CHAOS_LYAP_OK;
+  for (int i = 0; i < p.nseg && p.order_first && !rc; i++) rc = launch_order(p.part[i], s);
   if (p.nseg > 1 && (e = cudaEventRecord(h0->ev_fork, s)) != cudaSuccess)
     return cuda_fail(e, "batch fork");
-  int rc = CHAOS_LYAP_OK;
   for (int i = 0; i < p.nseg; i++) {
     const BatchPlan::Part &q = p.part[i];
     const cudaStream_t t = i ? h0->aux_stream[i - 1] : s;
     if (i && (e = cudaStreamWaitEvent(t, h0->ev_fork, 0)) != cudaSuccess)
       return cuda_fail(e, "batch fork");
-    if (!rc && q.a.order) {
-      rc = chaos::launch_order_longest_first(q.a.t_avg_per_point, q.a.P,
-                                             const_cast<int32_t *>(q.a.order), q.scratch, t);
-      if (rc) rc = cuda_fail((cudaError_t)rc, "order launch");
-    }
+    if (!rc && !p.order_first) rc = launch_order(q, t);
     if (!rc) rc = launch_part(p, q, t);
     // join even after a failed launch, so that a capture still ends cleanly
     if (i && ((e = cudaEventRecord(h0->ev_join[i - 1], t)) != cudaSuccess ||
