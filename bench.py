@@ -450,6 +450,7 @@ def measure_batch(a, rank, world, local, nsteps, nwarm, unbatched=True):
     total_points = sum(pt[1].shape[0] for pt in parts)
     stream = torch.cuda.Stream(dev)
     graph = cl.BatchGraph(parts)
+    batch_launches = parts[0][0].launches()  # of one replay
     peak = cl.fma_peak_tflops(local, "fp32", 1.0)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     with torch.cuda.stream(stream):
@@ -539,8 +540,7 @@ def measure_batch(a, rank, world, local, nsteps, nwarm, unbatched=True):
                    "form": {name: ("one point per group of four lanes"
                                    if form_of(name).startswith("split") else
                                    "one point per lane") for name in BATCH}},
-        # per segment: four kernels of the longest-first order and the sweep
-        "gpu_launches": nsteps * 5 * len(BATCH), "clocks": clk,
+        "gpu_launches": nsteps * batch_launches, "clocks": clk,
         "roofline": {"bound": "fp32_fma", "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                      "peak_source": "measured in-process (FMA-chain kernel)"},
@@ -751,6 +751,7 @@ def run_sweep_bench(a, w, rank, world, local):
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         elapsed_ms, kernel_ms = t.tolist()
 
+    launches = sw.launches()  # of one timed run
     total_points = P * a.steps * world
     value = total_points / (elapsed_ms * 1e-3)
     steps_np = steps.cpu().numpy()
@@ -856,10 +857,7 @@ def run_sweep_bench(a, w, rank, world, local):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": w["dtype"], "data": "synthetic (seeded grid and jitter)",
         "config": config_of(a, w, extra={"launch": tuned}),
-        # persistent sweeps of more than 1.5 waves: the transients, four kernels of
-        # the longest-first order and the averaging phases; otherwise one kernel
-        "gpu_launches": a.steps * (6 if tuned.get("schedule") == "persistent" and P >= 120_000
-                                   else 1),
+        "gpu_launches": a.steps * launches,
         "clocks": clk,
         "roofline": {"bound": "fp32_fma" if w["precision"] == "fp32" else "fp64_fma",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",

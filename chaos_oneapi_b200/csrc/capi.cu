@@ -155,6 +155,7 @@ struct chaos_lyap_handle {
   int block = 0;
   int schedule = CHAOS_SCHED_PERSISTENT;
   int variant = 0;  // kernel variant (chaos_lyap_desc.variant; autotuned)
+  int32_t launches = 0;  // kernels of the last run (chaos_lyap_get_launches)
   cudaStream_t own_stream = nullptr;
   cudaStream_t last_stream = nullptr;
   unsigned long long *queue = nullptr;  // point counters: persistent sweep / batch segments
@@ -489,7 +490,7 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
                    double t_transient_override, int64_t P_full = 0, int64_t stride = 1) {
   const chaos_lyap_desc &d = h->d;
   const ModelInfo *m = h->model;
-  int rc;
+  int rc, launches = 1;
   if (d.precision == CHAOS_PREC_COMPAT_FP64) {
     chaos::CompatArgs a{};
     a.P = P;
@@ -557,6 +558,7 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
               return cuda_fail((cudaError_t)rc, "kernel launch");
             if (!rc) {
               h->last_stream = s;
+              h->launches = 2 + chaos::kOrderKernels;
               return CHAOS_LYAP_OK;
             }
             a.resume = chaos::Resume{};
@@ -569,6 +571,7 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
         rc = chaos::launch_order_longest_first(a.t_avg_per_point, P, h->order, h->order_scratch, s);
         if (rc) return cuda_fail((cudaError_t)rc, "order launch");
         a.order = h->order;
+        launches += chaos::kOrderKernels;
       }
     }
     if (m->dim > 4) rc = chaos::launch_l96_warp(integ, prec, a, 0, s);
@@ -580,6 +583,7 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
                 m->name);
   if (rc != 0) return cuda_fail((cudaError_t)rc, "kernel launch");
   h->last_stream = s;
+  h->launches = launches;
   return CHAOS_LYAP_OK;
 }
 
@@ -992,6 +996,9 @@ static int enqueue_batch(const BatchPlan &p, chaos_lyap_handle *h0, cudaStream_t
               (e = cudaStreamWaitEvent(s, h0->ev_join[i - 1], 0)) != cudaSuccess))
       return cuda_fail(e, "batch join");
   }
+  h0->launches = 0;
+  for (int i = 0; i < p.nseg && !rc; i++)
+    if (p.part[i].a.P > 0) h0->launches += 1 + (p.part[i].a.order ? chaos::kOrderKernels : 0);
   return rc;
 }
 
@@ -1130,12 +1137,19 @@ int chaos_lyap_trajectory(chaos_lyap_handle *h, int64_t P, const double *params,
     return fail(CHAOS_LYAP_EUNSUPPORTED, "no trajectory kernel for model %s", m->name);
   if (rc) return cuda_fail((cudaError_t)rc, "trajectory launch");
   h->last_stream = (cudaStream_t)stream;
+  h->launches = 1;
   return CHAOS_LYAP_OK;
 }
 
 int chaos_lyap_get_variant(chaos_lyap_handle *h, int32_t *variant) {
   if (!h || !variant) return fail(CHAOS_LYAP_EINVAL, "null argument");
   *variant = h->variant;
+  return CHAOS_LYAP_OK;
+}
+
+int chaos_lyap_get_launches(chaos_lyap_handle *h, int32_t *kernels) {
+  if (!h || !kernels) return fail(CHAOS_LYAP_EINVAL, "null argument");
+  *kernels = h->launches;
   return CHAOS_LYAP_OK;
 }
 

@@ -89,6 +89,7 @@ struct AdaptiveArgs {
 // Longest-first hand-out order (order.cu): order = a permutation of [0, P)
 // by decreasing t_avg (bucketed); scratch holds kOrderScratchBytes.
 constexpr int kOrderBuckets = 1024;
+constexpr int kOrderKernels = 4;  // launches of an ordering
 constexpr size_t kOrderScratchBytes = 2 * sizeof(unsigned long long) + kOrderBuckets * sizeof(unsigned int);
 int launch_order_longest_first(const double *t_avg, int64_t P, int32_t *order, void *scratch,
                                cudaStream_t s);

@@ -240,6 +240,13 @@ class Sweep:
         check(lib.chaos_lyap_get_variant(self._h, ctypes.byref(v)))
         return v.value
 
+    def launches(self) -> int:
+        """Kernels that the last run (or, for a batch's first handle, the last
+        batch) enqueued: chaos_lyap_get_launches."""
+        v = ctypes.c_int32()
+        check(lib.chaos_lyap_get_launches(self._h, ctypes.byref(v)))
+        return v.value
+
 
 def cuda_lyapunov(task_num, is_qr, is_var, inits, close_points, dimension, model, params,
                   params_dim, eps, step, lyap_exps, exps_num, time_skip, time_skip_clp,

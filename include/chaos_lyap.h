@@ -274,6 +274,13 @@ int chaos_lyap_trajectory(chaos_lyap_handle *h, int64_t P, const double *params,
 /* The kernel variant in use (desc.variant, or the autotuner's choice). */
 int chaos_lyap_get_variant(chaos_lyap_handle *h, int32_t *variant);
 
+/* Kernels that the handle's last run enqueued: 1 for a sweep of one launch, 6 for
+ * one of two (transients, four of the hand-out order, averaging phases), 5 for a
+ * persistent sweep of points with averaging times of their own; for a batch, or a
+ * batch graph when it was created, all segments' together, on the first
+ * segment's handle. */
+int chaos_lyap_get_launches(chaos_lyap_handle *h, int32_t *kernels);
+
 /* Drop-in for the reference launcher cudaLyapunov (cuda/lyapunov.dp.hpp:10-17)
  * with the same argument meaning, DEVICE pointers, point-major layout:
  *   - the model is named instead of passed as three device function
