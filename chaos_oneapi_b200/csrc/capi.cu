@@ -414,23 +414,33 @@ static int ensure_order(chaos_lyap_handle *h, int64_t P) {
   return CHAOS_LYAP_OK;
 }
 
-// A persistent sweep (one lane or one warp per point) runs as two launches -- all transients, then the
-// averaging phases, those expected to take longest first -- when its points
-// are more than the GPU holds at once (otherwise every point starts at once and
-// the order cannot matter; just above one wave the run is its longest points
-// either way) but few enough waves that the end of the run, where lanes wait
-// for the longest points started last, is a sizeable part of it.  Needs a
-// transient (it is what predicts the cost); the buffers take 48-92 bytes per
-// point (Lorenz-96: 344-668).  One launch -> two, B200: 256^2 Lorenz points in
-// FP64 (1.7 waves) 245 -> 195 ms; FP32 Lorenz, 152k points (2 waves) 62 -> 47 ms,
-// 300k 103 -> 85 ms, 1024^2 (14 waves) 309 -> 275 ms; FP32 Rossler, whose
-// longest points take twice the mean, 152k points 82 -> 77 ms; at 1.1 waves of
-// it 55 -> 52 ms.
+// A persistent sweep (one lane or one warp per point) runs as two launches -- all
+// transients, then the averaging phases, those expected to take longest first --
+// when its points are more than the GPU holds at once (otherwise every point starts
+// at once and the order cannot matter).  Needs a transient, which is what predicts
+// the cost, of any length: t_transient / t_avg 0.1 to 60, points in the map's order
+// or shuffled, 1.55 to 31 waves: 0.99 (hyper-Rossler, 0.1, which gains nothing) to
+// 2.7 times as fast as one launch, the longer the transient the more.  The buffers
+// take 48-92 bytes per point (Lorenz-96: 344-668).  One launch -> two, B200: 256^2
+// Lorenz points in FP64 (1.7 waves) 245 -> 195 ms; FP32 Lorenz, 152k points (2 waves)
+// 62 -> 47 ms, 300k 103 -> 85 ms, 1024^2 (14 waves) 309 -> 279 ms; FP32 Rossler, whose
+// longest points take twice the mean, 152k points 82 -> 77 ms.
+//
+// From 1.5 waves on, because a lane renormalises with its warp, so that results
+// move with the grouping of the points, by less than the method's own error but
+// far on chaotic cells.  Just above one wave nearly every warp of a one-launch
+// sweep holds the same points in every run and the results repeat; two launches
+// would group all of them anew (FP32 Rossler, 1.1 waves: 55 -> 52 ms, and four times
+// the difference of two runs of one launch).  At 1.55 waves that is 1.26 times (root
+// mean square 0.044 against 0.035), with the same errors against the exact exponents
+// (tests/test_gpu_two_phase_models.py).
 constexpr double kTwoPhaseMinWaves = 1.5;
 // The warp-per-point form renormalises each point by itself, so its results do
 // not depend on the order at all: from the first point that has to wait.
 // Lorenz-96, 64^2 points (1.7 waves): 116 -> 94 ms.
 constexpr double kTwoPhaseMinWavesWarp = 1.0;
+// Up to here the buffers stay below 120 MB, within what the pool keeps; the gain of
+// a short transient is down to 1.06 (FP32) and 1.03 (FP64) at 31 waves.
 constexpr int64_t kTwoPhaseMaxWaves = 32;
 
 // Buffers of one two-launch sweep of P points, from the pool and back to it in
