@@ -552,6 +552,9 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
       a.queue = h->queue;
       a.queue_stride = chaos::queue_stride_for(P);
       const bool warp = m->dim > 4;
+      // (also where this run takes two launches: a capture of the same call takes one
+      // and cannot allocate)
+      if (a.t_avg_per_point && !warp && (rc = ensure_order(h, P))) return rc;
       if (!split && a.t_transient > 0) {
         const int64_t held = warp ? chaos::l96_resident(integ, prec, d.k)
                                   : chaos::adaptive_resident(m->id, integ, prec, block, variant);
@@ -576,8 +579,7 @@ static int enqueue(chaos_lyap_handle *h, int64_t P, const double *params, double
           }
         }
       }
-      if (a.t_avg_per_point && m->dim <= 4) {  // longest averaging time first
-        if ((rc = ensure_order(h, P))) return rc;
+      if (a.t_avg_per_point && !warp) {  // longest averaging time first
         rc = chaos::launch_order_longest_first(a.t_avg_per_point, P, h->order, h->order_scratch, s);
         if (rc) return cuda_fail((cudaError_t)rc, "order launch");
         a.order = h->order;

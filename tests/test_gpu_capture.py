@@ -81,3 +81,26 @@ def test_sweep_beside_an_open_capture(lib, mode, own_thread):
     assert not errors
     assert (z == 2).all() and (status == 0).all()
     sw.close()
+
+
+def test_sweep_of_own_times_captured_after_a_run(lib):
+    """A run makes what a later capture of the same call needs, also where the
+    run itself takes two launches and the captured one one."""
+    import torch
+    P = 60_001
+    sw, p, x, spec, status, _, _ = _part(lib, torch, "lorenz", P)
+    t_avg = torch.linspace(0.5, 4.0, P, dtype=torch.float64, device="cuda")
+    sw.run(p, x, spec, status, t_avg=t_avg)
+    torch.cuda.synchronize()
+    want = spec.clone()
+    spec.zero_()
+    status.fill_(-1)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        sw.run(p, x, spec, status, t_avg=t_avg)
+    g.replay()
+    torch.cuda.synchronize()
+    assert (status == 0).all()
+    # regular cells: both within the integration error, some 1e3 rtol
+    assert (spec - want).abs().max() < 1e3 * KW["rtol"]
+    sw.close()
