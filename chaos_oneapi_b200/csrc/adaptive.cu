@@ -50,7 +50,7 @@ __device__ __forceinline__ void lane_begin(Lane<M, K, R, INTEG> &L, const Adapti
 // is voted per warp: when any lane is due, every lane past its transient
 // renormalises in the same pass.
 // MINB: resident 128-thread blocks per SM the kernel is compiled for (a
-// register cap: 3 -> 168 registers, 4 -> 128, 5 -> 96 with a few spills); the
+// register cap: 3 -> at most 168 registers, 4 -> 128, 5 -> 96 with a few spills); the
 // autotuner picks the variant, except in batches (kBatchVariant).
 // RESUME: the averaging phases of points whose transients have run.
 template <class M, int K, class R, int INTEG, int MINB, bool RESUME = false>

@@ -789,25 +789,24 @@ int chaos_lyap_autotune_map(chaos_lyap_handle *h, int64_t P, int64_t sample,
 //
 // An FP32 batch of few waves whose points have averaging times of their own is as
 // long as its longest points' chains of steps, and a step takes longer the more
-// warps share its scheduler: its one-lane segments run in the build of three
-// blocks per SM instead of four, whichever segments share an SM.  Averaging times T
-// to 4 T, one kernel for all / four blocks / three: 65,536 hyper-Rossler and 65,536
-// Lorenz points 307 / 371 / 305 ms, with as many Chua points 383 / 391 / 298 ms;
-// 150,000 Lorenz points (2 waves) 8.0 / 6.8 / 6.8 ms.  From kBatchFewWaves waves of
-// the four-block build on its throughput counts: 300,000 Lorenz points (4 waves)
+// warps share its scheduler: its one-lane segments run in the build of up to 168
+// registers, three blocks per SM instead of four for the models that use more than
+// 128 (hyper-Rossler 164, Shimizu 143, Lorenz 137; Rossler and Chua still fit four
+// times).  Averaging times T to 4 T, one kernel for all / 128 registers / 168:
+// 65,536 hyper-Rossler and as many Lorenz points 307 / 371 / 305 ms, with as many
+// Chua points 383 / 391 / 298 ms; 150,000 Lorenz points (2 waves) 8.0 / 6.8 / 6.8 ms.
+// From kBatchFewWaves waves on throughput counts: 300,000 Lorenz points (4 waves)
 // 15.2 / 12.3 / 12.9 ms.  Segments that lie apart gain nothing: 19,891 Lorenz and as
 // many Rossler points (0.5 waves) 4.1 / 3.0-3.3 / 3.3 ms, eight segments of 4,096
 // 3.6 / 1.4 / 1.5 ms; beside a split segment they meet sooner (3 x 128^2 points, 0.4
-// waves of them: 36.1 / 27.8 / 26.5 ms).
+// waves of them: 36.1 / 27.6 / 26.4 ms).
 constexpr double kBatchFewWaves = 3.0, kBatchApartWaves = 0.6, kBatchApartWavesSplit = 0.25;
 // Such a batch of one segment takes two blocks per SM while its points come out
-// even over them: up to kBatchSoloWaves times the build's lanes.  One kernel / four
-// blocks / three / two: hyper-Rossler, 39,782 points 252 / 278 / 294 / 223 ms, 65,546
-// points 280 / 384 / 297 / 221, 77,670 points 291 / 387 / 299 / 227; Lorenz, 39,782
-// points 3.5 / 4.0 / 3.9 / 3.0, 77,670 points 4.6 / 5.2 / 4.1 / 4.1, 100,000 points 5.6
-// / 5.4 / 4.7 / 5.2 ms.
-constexpr int kBatchSoloLanes = 256;  // per SM
-constexpr double kBatchSoloWaves = 1.5;
+// even over them, up to kBatchSoloPoints.  One kernel / 128 registers / 168 / two
+// blocks: hyper-Rossler, 39,782 points 252 / 278 / 294 / 223 ms, 65,546 points 280 /
+// 384 / 297 / 221, 77,670 points 291 / 387 / 299 / 227; Lorenz, 39,782 points 3.5 / 4.0 /
+// 3.9 / 3.0, 77,670 points 4.6 / 5.2 / 4.1 / 4.1, 100,000 points 5.6 / 5.4 / 4.7 / 5.2 ms.
+constexpr int kBatchSoloLanes = 256, kBatchSoloPoints = 576;  // per SM
 // Among the one-lane segments those of fewer points are launched first: they
 // start whole beside a part of the larger ones, whose other points follow as
 // lanes become free.  If they do not all fit, the orders are made before the
@@ -951,7 +950,7 @@ static int build_batch(const chaos_lyap_segment *segs, int nseg, BatchPlan *plan
       plan->prec == chaos::kFP32 && waves < kBatchFewWaves &&
       (nseg == 1 || waves > (nsplit ? kBatchApartWavesSplit : kBatchApartWaves));
   plan->solo = plan->few_waves && nseg == 1 && nsplit == 0 && plan->part[0].a.order &&
-               lane_waves(*plan, true) <= kBatchSoloWaves;
+               plan->part[0].a.P <= (int64_t)kBatchSoloPoints * h0->sm_count;
   plan->order_first = nseg > 1 && nsplit == 0 && lane_waves(*plan, plan->few_waves) > 1.0;
   if (nseg > 1) {  // fork / join resources
     cudaError_t e = cudaSuccess;

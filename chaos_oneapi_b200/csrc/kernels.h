@@ -112,8 +112,8 @@ enum Precision : int32_t { kCompatFP64 = 0, kFP64 = 1, kFP32 = 2 };
 constexpr int kErrUnsupported = -1;
 
 int launch_compat(int model, const CompatArgs &a, int block, cudaStream_t s);
-// variant: 0 = 128-register build, 1 = 96-register build, kBatchVariant =
-// 168-register build (FP32 only); lanes_per_sm: a persistent launch takes at most
+// variant (FP32 only): builds of at most 128 registers (0), 96 (1) and 168
+// (kBatchVariant); lanes_per_sm: a persistent launch takes at most
 // so many (0: all that fit)
 constexpr int kBatchVariant = 2;
 int launch_adaptive(int model, int integrator, int precision, const AdaptiveArgs &a, int block,

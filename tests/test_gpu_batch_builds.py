@@ -1,6 +1,7 @@
 """FP32 batches of points with averaging times of their own: the launch forms
-they run in (three blocks per SM in a few waves, two in a batch of one segment,
-the sweeps' own build from three waves on) against sweeps of the same points."""
+they run in (a build of up to 168 registers in a few waves, on two blocks per SM in
+a batch of one segment; the sweeps' own build from three waves on) against sweeps
+of the same points."""
 import numpy as np
 import pytest
 
@@ -30,7 +31,7 @@ def _inputs(model, P, block, integrator):
 @pytest.mark.parametrize("integrator", ["dopri5", "dverk65"])
 @pytest.mark.parametrize("spec", [
     (("lorenz", 3000),), (("rossler", 50_001),), (("hyper_rossler", 50_001),),  # two blocks per SM
-    (("shimizu", 120_001),), (("lorenz", 240_001),),                           # three; own build
+    (("shimizu", 120_001),), (("lorenz", 240_001),),                           # own build last
     (("chua", 40_001), ("lorenz", 257), ("hyper_rossler", 30_001), ("shimizu", 0)),
     (("chua", 1001), ("rossler", 997))], ids=lambda s: "-".join(f"{m}{n}" for m, n in s))
 @pytest.mark.parametrize("block", [128, 64])
