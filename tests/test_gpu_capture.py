@@ -92,15 +92,18 @@ def test_sweep_of_own_times_captured_after_a_run(lib):
     t_avg = torch.linspace(0.5, 4.0, P, dtype=torch.float64, device="cuda")
     sw.run(p, x, spec, status, t_avg=t_avg)
     torch.cuda.synchronize()
-    want = spec.clone()
+    assert sw.launches() == 6
     spec.zero_()
     status.fill_(-1)
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
         sw.run(p, x, spec, status, t_avg=t_avg)
+    assert sw.launches() == 5
     g.replay()
     torch.cuda.synchronize()
     assert (status == 0).all()
-    # regular cells: both within the integration error, some 1e3 rtol
-    assert (spec - want).abs().max() < 1e3 * KW["rtol"]
+    # the exponents add up to the trace -(sigma + 1 + beta) on every cell, also
+    # beside a separatrix, where single exponents depend on the grouping; to the
+    # integration error, some 1e3 rtol
+    assert (spec.sum(1) + p[:, 0] + 1 + p[:, 2]).abs().max() < 1e3 * KW["rtol"]
     sw.close()
